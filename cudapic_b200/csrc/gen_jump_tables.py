@@ -1,9 +1,9 @@
-"""Generates jump_tables.inc: the GF(2) matrices of J^(2^b), b = 4..27, where
+"""Generates jump_tables.inc: the GF(2) matrices of J^(2^b), b = 0..27, where
 J is the xoshiro128+ jump() (advance by 2^64 steps, Rust-CUDA/src/main.rs:
 1452, 1473-1487).  xoshiro128+ is linear over GF(2), so J is a 128 x 128 bit
 matrix whose column j is jump() applied to the unit state e_j; its powers by
-repeated squaring let one GPU thread compute stream 16*m = J^(16 m) master
-directly instead of performing 16 m sequential jumps.
+repeated squaring let a CTA form stream k = J^k master of its first slot from
+the set bits of k instead of performing k sequential jumps.
 
 Usage: python gen_jump_tables.py OUT_FILE   (run by cudapic_b200/build.py)
 """
@@ -11,8 +11,8 @@ import sys
 
 JUMP = (0x8764000B, 0xF542D2D3, 0x6FA035C3, 0x77F2DB5B)
 M32 = 0xFFFFFFFF
-FIRST_LEVEL = 4   # streams are produced in chunks of 2^4 consecutive jumps
-LEVELS = 24       # levels 4..27: up to 2^28 streams
+FIRST_LEVEL = 0   # level b of the table is J^(2^(b + FIRST_LEVEL))
+LEVELS = 28       # levels 0..27: up to 2^28 streams
 
 
 def _next(s):
@@ -59,19 +59,18 @@ def jump_power_columns():
         s[j // 32] = 1 << (j % 32)
         unit.append(_to_int(_jump(s)))
     levels = [unit]
-    for _ in range(FIRST_LEVEL + LEVELS - 1):
+    for _ in range(LEVELS - 1):
         m = levels[-1]
         levels.append([_matvec(m, c) for c in m])
-    return levels[FIRST_LEVEL:FIRST_LEVEL + LEVELS]
+    return levels
 
 
 def main(out_path):
     tables = jump_power_columns()
     lines = ["// generated by gen_jump_tables.py -- do not edit",
-             "// c_jump_pow[l][j] = column j of J^(2^(l+%d)) as (s0, s1, s2, s3)" % FIRST_LEVEL,
-             "#define CUDAPIC_JUMP_FIRST_LEVEL %d" % FIRST_LEVEL,
+             "// d_jump_pow[l][j] = column j of J^(2^l) as (s0, s1, s2, s3)",
              "#define CUDAPIC_JUMP_LEVELS %d" % LEVELS,
-             "__constant__ uint4 c_jump_pow[%d][128] = {" % LEVELS]
+             "__device__ const uint4 d_jump_pow[%d][128] = {" % LEVELS]
     for cols in tables:
         row = []
         for c in cols:

@@ -5,12 +5,25 @@
 // O(128 n) sequential jumps); xoshiro128p_test_wrapper, :1341-1357.
 //
 // Seeding on the GPU: xoshiro128+ is linear over GF(2), so stream k = J^k m
-// (m = master state, J = the 128x128 bit matrix of one jump).  The matrices
-// J^(2^b), b = 4..27, are generated at build time (gen_jump_tables.py) into
-// constant memory.  Thread t produces streams 16t..16t+15: it forms J^(16t) m
-// from the set bits of 16t (one 128-column matrix-vector product per level,
-// all lanes reading the same column: a constant-cache broadcast), then
-// applies 15 sequential jumps.  Bit-identical to the sequential host loop.
+// (m = master state, J = the 128x128 bit matrix of one jump); the matrices
+// J^(2^l), l = 0..27, are generated at build time (gen_jump_tables.py).
+// CTA c produces the streams [k0, k0 + 256 R), k0 = 256 R c:
+//  1. one warp forms J^k0 m from the set bits of k0, four matrix columns per
+//     lane and an XOR reduction over the warp; meanwhile the other warps
+//     build the product table of step 3;
+//  2. the CTA doubles that state to 256 consecutive ones (t + 2^l from t with
+//     the matrix of level l, one warp per product: 255 products in all);
+//  3. each thread then steps by J^256, R - 1 times, storing one state per
+//     step: the stores of a warp are consecutive.  The product is 22 table
+//     lookups (6 bits of the state each, 128 B of shared memory per row: the
+//     16-byte product repeated for 8 lanes, so that the 8 lanes which a
+//     128-bit shared load serves together always use different banks).
+// Bound by the shared loads: 22 x 4 wavefronts per 32 streams and SM.  A
+// product by masked columns (128 x 6 instructions) was bound by instructions
+// and stored 16 consecutive streams per thread, uncoalesced: 2 097 155 streams
+// took 277 us, now 35 us (byte tables of 64 KB have fewer lookups but about
+// 2.7 lanes per bank; nibble tables 32 lookups).
+// Bit-identical to the sequential host loop.
 #include "common.cuh"
 #include "detmath.cuh"
 #include "internal.h"
@@ -21,64 +34,127 @@
 
 namespace cudapic {
 
-constexpr uint32_t SEED_CHUNK = 1u << CUDAPIC_JUMP_FIRST_LEVEL;
+constexpr int SEED_THREADS = 256;
+constexpr int SEED_WARPS = SEED_THREADS / 32;
+constexpr int SEED_LEVEL = 8;             // a thread steps by J^(2^8) = J^SEED_THREADS
+constexpr int SEED_GROUPS = 22;           // 6-bit groups of a 128-bit state (the last one: 2 bits)
+constexpr uint32_t SEED_ROWS = 21u * 64u + 4u;
+constexpr size_t SEED_TABLE_BYTES = (size_t)SEED_ROWS * 128;
+static_assert((1 << SEED_LEVEL) == SEED_THREADS, "a step covers the CTA's threads");
 
-__device__ __forceinline__ uint4 jump_seq(uint4 s) {
-    const uint32_t J[4] = {0x8764000bu, 0xf542d2d3u, 0x6fa035c3u, 0x77f2db5bu};
-    uint4 acc = make_uint4(0, 0, 0, 0);
-    Xoshiro128p r{s.x, s.y, s.z, s.w};
+__device__ __forceinline__ void xor4(uint4 &a, const uint4 &b) {
+    a.x ^= b.x;
+    a.y ^= b.y;
+    a.z ^= b.z;
+    a.w ^= b.w;
+}
+
+// The calling lane's four columns (4 lane .. 4 lane + 3) of level l.
+__device__ __forceinline__ void seed_columns(int l, int lane, uint4 (&c)[4]) {
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
+    for (int q = 0; q < 4; ++q) c[q] = __ldg(&d_jump_pow[l][4 * lane + q]);
+}
+
+// Matrix-vector product by one warp (all lanes hold the state s and their
+// four columns c); every lane gets the product.
+__device__ __forceinline__ uint4 seed_product(const uint4 &s, const uint4 (&c)[4], int lane) {
+    const uint32_t word = lane < 16 ? (lane < 8 ? s.x : s.y) : (lane < 24 ? s.z : s.w);
+    const uint32_t bits = word >> ((4 * lane) & 31);
+    uint4 acc = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-        for (int b = 0; b < 32; ++b) {
-            if (J[w] & (1u << b)) {
-                acc.x ^= r.s0;
-                acc.y ^= r.s1;
-                acc.z ^= r.s2;
-                acc.w ^= r.s3;
-            }
-            r.next();
-        }
+    for (int q = 0; q < 4; ++q) {
+        const uint32_t m = 0u - ((bits >> q) & 1u);
+        acc.x ^= c[q].x & m;
+        acc.y ^= c[q].y & m;
+        acc.z ^= c[q].z & m;
+        acc.w ^= c[q].w & m;
+    }
+    acc.x = __reduce_xor_sync(0xffffffffu, acc.x);
+    acc.y = __reduce_xor_sync(0xffffffffu, acc.y);
+    acc.z = __reduce_xor_sync(0xffffffffu, acc.z);
+    acc.w = __reduce_xor_sync(0xffffffffu, acc.w);
+    return acc;
+}
+
+// Rows first, first + stride, ...: row 64 g + v is the XOR of the columns
+// 6 g + i of level SEED_LEVEL over the set bits i of v, repeated 8 times (in
+// an order rotated by the lane: conflict-free stores).
+__device__ __forceinline__ void seed_fill_table(uint4 *tab, uint32_t first, uint32_t stride, int lane) {
+    for (uint32_t row = first; row < SEED_ROWS; row += stride) {
+        const uint32_t g = row >> 6, v = row & 63u;
+        uint4 e = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (uint32_t i = 0; i < 6; ++i)
+            if (v >> i & 1u) xor4(e, __ldg(&d_jump_pow[SEED_LEVEL][6u * g + i]));  // g = 21: v < 4
+#pragma unroll
+        for (uint32_t r = 0; r < 8; ++r) tab[row * 8u + ((r + (uint32_t)lane) & 7u)] = e;
+    }
+}
+
+// J^SEED_THREADS s from the table (mine: the table at this lane's copy).
+__device__ __forceinline__ uint4 seed_step(const uint4 &s, const uint4 *mine) {
+    const uint32_t w[5] = {s.x, s.y, s.z, s.w, 0u};
+    uint4 acc = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int g = 0; g < SEED_GROUPS; ++g) {
+        const int bit = 6 * g, k = bit >> 5, sh = bit & 31;
+        const uint32_t v = __funnelshift_r(w[k], w[k + 1], sh) & 63u;  // the last group reads zeros past bit 127
+        xor4(acc, mine[(64u * (uint32_t)g + v) * 8u]);
     }
     return acc;
 }
 
-__global__ void __launch_bounds__(256)
-    seed_streams_kernel(uint4 master, uint32_t n, uint32_t *__restrict__ r0, uint32_t *__restrict__ r1,
-                        uint32_t *__restrict__ r2, uint32_t *__restrict__ r3) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t k0 = (uint64_t)t * SEED_CHUNK;
-    if (k0 >= n) return;
-    uint4 s = master;
-    for (int l = 0; l < CUDAPIC_JUMP_LEVELS; ++l) {
-        const uint32_t use = 0u - (uint32_t)((k0 >> (l + CUDAPIC_JUMP_FIRST_LEVEL)) & 1u);
-        uint4 acc = make_uint4(0, 0, 0, 0);
-        const uint32_t words[4] = {s.x, s.y, s.z, s.w};
+__global__ void __launch_bounds__(SEED_THREADS)
+    seed_streams_kernel(uint4 master, uint32_t n, uint32_t per_thread, uint32_t *__restrict__ r0,
+                        uint32_t *__restrict__ r1, uint32_t *__restrict__ r2, uint32_t *__restrict__ r3) {
+    extern __shared__ __align__(128) unsigned char seed_smem[];
+    uint4 *tab = reinterpret_cast<uint4 *>(seed_smem);  // [SEED_ROWS][8] (per_thread > 1)
+    __shared__ uint4 st[SEED_THREADS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t k0 = blockIdx.x * (SEED_THREADS * per_thread);  // < n <= 2^28
+    if (warp == 0) {
+        uint4 s = master, c[4];
+        uint32_t left = k0;
+        if (left) seed_columns(__ffs(left) - 1, lane, c);
+        while (left) {  // the next level's columns are fetched during this level's product
+            left &= left - 1u;
+            uint4 next[4] = {};
+            if (left) seed_columns(__ffs(left) - 1, lane, next);
+            s = seed_product(s, c, lane);
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-#pragma unroll 8
-            for (int b = 0; b < 32; ++b) {
-                const uint32_t m = 0u - ((words[w] >> b) & 1u);
-                const uint4 c = c_jump_pow[l][w * 32 + b];
-                acc.x ^= c.x & m;
-                acc.y ^= c.y & m;
-                acc.z ^= c.z & m;
-                acc.w ^= c.w & m;
-            }
+            for (int q = 0; q < 4; ++q) c[q] = next[q];
         }
-        s.x = (acc.x & use) | (s.x & ~use);
-        s.y = (acc.y & use) | (s.y & ~use);
-        s.z = (acc.z & use) | (s.z & ~use);
-        s.w = (acc.w & use) | (s.w & ~use);
+        if (lane == 0) st[0] = s;
+    } else if (per_thread > 1) {
+        seed_fill_table(tab, (uint32_t)(tid - 32), SEED_THREADS - 32, lane);
     }
-    for (uint32_t c = 0; c < SEED_CHUNK; ++c) {
-        const uint64_t k = k0 + c;
+    uint4 c[4];
+    seed_columns(0, lane, c);
+#pragma unroll
+    for (int l = 0; l < SEED_LEVEL; ++l) {
+        uint4 next[4] = {};
+        if (l + 1 < SEED_LEVEL) seed_columns(l + 1, lane, next);
+        __syncthreads();
+        for (int t = warp; t < (1 << l); t += SEED_WARPS) {
+            const uint4 p = seed_product(st[t], c, lane);
+            if (lane == 0) st[t + (1 << l)] = p;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) c[q] = next[q];
+    }
+    __syncthreads();
+    uint4 s = st[tid];
+    const uint4 *mine = tab + (lane & 7);
+    uint64_t k = (uint64_t)k0 + tid;
+    for (uint32_t r = 0;;) {
         if (k >= n) break;
         r0[k] = s.x;
         r1[k] = s.y;
         r2[k] = s.z;
         r3[k] = s.w;
-        if (c + 1 < SEED_CHUNK && k + 1 < n) s = jump_seq(s);
+        if (++r == per_thread) break;
+        s = seed_step(s, mine);
+        k += SEED_THREADS;
     }
 }
 
@@ -151,12 +227,20 @@ extern "C" int cudapic_xoshiro128_seed_streams(const uint32_t master[4], uint32_
     CUDAPIC_REQUIRE(master && rng0 && rng1 && rng2 && rng3, "xoshiro128_seed_streams: null pointer");
     CUDAPIC_REQUIRE((master[0] | master[1] | master[2] | master[3]) != 0u,
                     "xoshiro128_seed_streams: master state must not be all zero");
-    CUDAPIC_REQUIRE((uint64_t)n <= (1ull << (CUDAPIC_JUMP_FIRST_LEVEL + CUDAPIC_JUMP_LEVELS)),
-                    "xoshiro128_seed_streams: n > 2^28");
+    CUDAPIC_REQUIRE((uint64_t)n <= (1ull << CUDAPIC_JUMP_LEVELS), "xoshiro128_seed_streams: n > 2^28");
     if (n == 0) return CUDAPIC_OK;
-    const uint32_t threads = (n + SEED_CHUNK - 1) / SEED_CHUNK;
     const uint4 m = make_uint4(master[0], master[1], master[2], master[3]);
-    seed_streams_kernel<<<(threads + 255) / 256, 256, 0, (cudaStream_t)stream>>>(m, n, rng0, rng1, rng2, rng3);
+    // one CTA per SM, each a contiguous range of 256 x per_thread streams; up
+    // to one stream per thread (n <= 256 SMs) nothing is stepped: no table
+    const uint32_t step = (uint32_t)sm_count() * SEED_THREADS;
+    const uint32_t per_thread = (n + step - 1) / step;
+    const uint32_t block = SEED_THREADS * per_thread;
+    const size_t smem = per_thread > 1 ? SEED_TABLE_BYTES : 0;
+    if (smem)
+        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(seed_streams_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                      (int)smem), "cudaFuncSetAttribute(xoshiro128_seed_streams)"));
+    seed_streams_kernel<<<(n + block - 1) / block, SEED_THREADS, smem, (cudaStream_t)stream>>>(m, n, per_thread, rng0,
+                                                                                              rng1, rng2, rng3);
     return check_launch("xoshiro128_seed_streams");
 }
 

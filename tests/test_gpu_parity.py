@@ -62,6 +62,18 @@ def test_seed_streams_bit_exact(K, oracle, n):
         assert np.array_equal(host(p), r)
 
 
+@pytest.mark.parametrize("per,extra", [(0, 255), (0, 256), (0, 257), (1, -1), (1, 0), (1, 1), (2, 0), (2, 1), (3, -77)])
+def test_seed_streams_at_block_edges(K, oracle, per, extra):
+    # CTAs of 256 threads, one per SM, each thread `per` streams: the ends of a CTA's and of the grid's range
+    import torch
+    n = per * 256 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    master = [0x9E3779B9, 0, 0x80000000, 1]
+    planes = [zeros(n + 4, np.uint32) for _ in range(4)]
+    K.xoshiro128_seed_streams(master, n, *planes)
+    for p, r in zip(planes, oracle.seed_streams(master, n)):
+        assert np.array_equal(host(p)[:n], r) and not host(p)[n:].any()
+
+
 @pytest.mark.parametrize("fn,lo,hi", [("exp", -40.0, 5.0), ("log", 1e-9, 1.0), ("sin", -10.0, 10.0),
                                       ("cos", -10.0, 10.0), ("tan", -1.5, 1.5), ("atan", -60.0, 60.0),
                                       ("acos", -1.0, 1.0), ("atan2", -4.0, 4.0)])
