@@ -94,9 +94,12 @@ int launch_poisson(const float *e_density, const float *i_density, float *pot, f
                    float *zero_a = nullptr, float *zero_b = nullptr);
 // Adjoint of launch_poisson's solve and field in FP64 (kernels_poisson.cu):
 // eb (field adjoint, cleared) -> neb, nib_acc (density adjoints, the ion one
-// accumulated unless reset_acc) and vbar += cosv * (pot0 adjoint).
+// accumulated unless reset_acc) and vbar += cosv * (pot0 adjoint), for `obs`
+// observables at once ([obs][n_g] arrays, vbar [obs]).
 int launch_poisson_adjoint(double *eb, double *neb, double *nib_acc, int reset_acc, double cosv, double *vbar,
-                           const cudapic_grid &g, cudaStream_t stream);
+                           int obs, const cudapic_grid &g, cudaStream_t stream);
+// Threads and nodes per thread (a power of two) of the one-CTA solves.
+void poisson_shape(uint32_t n_g, int &threads, int &per_thread);
 // FP64 solve and field from FP64 node sums (kernels_poisson.cu, the all-FP64
 // twin): pot0 from pot0_table[*step % n_t], *step advanced; measurement sums
 // may be null.

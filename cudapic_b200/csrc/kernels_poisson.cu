@@ -144,7 +144,8 @@ int launch_poisson_pt(const float *e_density, const float *i_density, float *pot
 // nib_acc = (reset_acc ? 0 : nib_acc) + e rho_bar (rho_bar = alpha lam inside,
 // the one-sided corrections at the electrodes), and
 // vbar += cosv (pb_0 - lam_1), pot0 = V cosv entering f_1 with a minus sign.
-// One CTA; eb is cleared for the next step.
+// One CTA per observable o = blockIdx.x (eb, neb, nib_acc [o][n_g], vbar
+// [o]); eb is cleared for the next step.
 template <int PT>
 __global__ void __launch_bounds__(POIS_MAX_THREADS)
     poisson_adjoint_kernel(double *__restrict__ eb, double *__restrict__ neb, double *__restrict__ nib_acc,
@@ -153,7 +154,12 @@ __global__ void __launch_bounds__(POIS_MAX_THREADS)
     double *eb_s = reinterpret_cast<double *>(smem_raw);  // n
     __shared__ double wsum[32];
     __shared__ double r_total_s, lam1_s;
+    grid_dep_wait();
     const int n = (int)g.n_g;
+    eb += (size_t)blockIdx.x * n;
+    neb += (size_t)blockIdx.x * n;
+    nib_acc += (size_t)blockIdx.x * n;
+    vbar += blockIdx.x;
     const int tid = threadIdx.x;
     for (int k = tid; k < n; k += blockDim.x) {
         eb_s[k] = eb[k];
@@ -226,28 +232,28 @@ __global__ void __launch_bounds__(POIS_MAX_THREADS)
 
 template <int PT>
 int launch_poisson_adjoint_t(double *eb, double *neb, double *nib_acc, int reset_acc, double cosv, double *vbar,
-                             const cudapic_grid &g, int threads, cudaStream_t stream) {
+                             int obs, const cudapic_grid &g, int threads, cudaStream_t stream) {
     const size_t smem = (size_t)g.n_g * sizeof(double);
     auto kern = poisson_adjoint_kernel<PT>;
     if (smem > 48 * 1024)
         CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                                  "cudaFuncSetAttribute(poisson_adjoint)"));
-    return launch_kernel("poisson_adjoint", kern, dim3(1), dim3(threads), smem, stream, eb, neb, nib_acc, reset_acc,
+    return launch_kernel("poisson_adjoint", kern, dim3(obs), dim3(threads), smem, stream, eb, neb, nib_acc, reset_acc,
                          cosv, vbar, g);
 }
 
 int launch_poisson_adjoint(double *eb, double *neb, double *nib_acc, int reset_acc, double cosv, double *vbar,
-                           const cudapic_grid &g, cudaStream_t stream) {
+                           int obs, const cudapic_grid &g, cudaStream_t stream) {
     if (g.n_g < 3 || g.n_g > (uint32_t)(POIS_MAX_THREADS * POIS_MAX_PER_THREAD))
         return fail(CUDAPIC_ERR_ARG, "poisson_adjoint: n_g outside 3..16384");
     int threads, pt;
     poisson_shape(g.n_g, threads, pt);
     switch (pt) {
-    case 1: return launch_poisson_adjoint_t<1>(eb, neb, nib_acc, reset_acc, cosv, vbar, g, threads, stream);
-    case 2: return launch_poisson_adjoint_t<2>(eb, neb, nib_acc, reset_acc, cosv, vbar, g, threads, stream);
-    case 4: return launch_poisson_adjoint_t<4>(eb, neb, nib_acc, reset_acc, cosv, vbar, g, threads, stream);
-    case 8: return launch_poisson_adjoint_t<8>(eb, neb, nib_acc, reset_acc, cosv, vbar, g, threads, stream);
-    default: return launch_poisson_adjoint_t<16>(eb, neb, nib_acc, reset_acc, cosv, vbar, g, threads, stream);
+    case 1: return launch_poisson_adjoint_t<1>(eb, neb, nib_acc, reset_acc, cosv, vbar, obs, g, threads, stream);
+    case 2: return launch_poisson_adjoint_t<2>(eb, neb, nib_acc, reset_acc, cosv, vbar, obs, g, threads, stream);
+    case 4: return launch_poisson_adjoint_t<4>(eb, neb, nib_acc, reset_acc, cosv, vbar, obs, g, threads, stream);
+    case 8: return launch_poisson_adjoint_t<8>(eb, neb, nib_acc, reset_acc, cosv, vbar, obs, g, threads, stream);
+    default: return launch_poisson_adjoint_t<16>(eb, neb, nib_acc, reset_acc, cosv, vbar, obs, g, threads, stream);
     }
 }
 

@@ -23,6 +23,19 @@
 //        n v at node N_G-1 (boundary node doubled, as the density), a smooth
 //        estimate of the counted flux of C/eduPIC.cc:651-658.
 //
+// Step kernels: one forward step is three launches -- the field (node sums to
+// densities, the solve, the step's marks: one CTA), the electrons (push,
+// collisions and the next step's deposit in one pass over the slots) and the
+// spawns -- and four more on an ion step.  At 2e5 particles every one of them
+// is a few microseconds of latency, so what counts is their number and that
+// programmatic dependent launch overlaps each one's launch with the previous
+// one's tail (every kernel waits before its first global access).  The
+// backward pass recomputes each checkpoint interval once and sweeps the
+// adjoints of both observables through it together: they share the tape, the
+// records and the collision Jacobians.  2e5 + 2e5 particles, 200 steps:
+// forward 3.6 ms, backward 10.2 ms (with seven launches per forward step, no
+// overlap and a recompute per observable: 8.5 and 32.7 ms).
+//
 // Adjoint kernels: push (field gather -> its adjoint scatters into the field
 // adjoint, FP64 shared-memory sums), collisions (Jacobians by forward-mode
 // tangents of the same scattering arithmetic, applied transposed), spawns
@@ -40,7 +53,10 @@
 #include "detmath.cuh"
 #include "internal.h"
 #include "mcc.cuh"
+#include "poisson.cuh"
+#include "push.cuh"
 #include "state_impl.h"
+#include "step.cuh"
 
 namespace cudapic {
 
@@ -52,7 +68,7 @@ constexpr uint32_t SENS_CHUNK = 1024;      // spawn-order chunk (one CTA of the 
 constexpr uint32_t NO_SPAWN = 0xFFFFFFFFu;
 constexpr uint32_t SPAWN_NOREC = 0xFFFFFFFEu;
 constexpr uint32_t NO_SLOT = 0xFFFFFFFFu;
-constexpr uint32_t SENS_DEP_Q = 20;
+constexpr uint32_t SENS_DEP_EPOCH = DEP_MAX_PER_COPY / SENS_THREADS;  // rounds of a CTA between drains
 constexpr uint32_t SENS_MAX_NG = 4096;
 
 // counters block
@@ -258,33 +274,88 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
 }
 
 // ------------------------------------------------------------------ forward
+// The CTA's deposit: 2^-20 fixed-point weights (push.cuh dep_add) in a 32-bit
+// shared histogram (five times the rate of 64-bit shared atomics), drained
+// into 64-bit sums before a node can overflow.  Dynamic shared memory:
+// [n_g] u64, [n_g] u32.  The node sums are exact, so neither the order nor the
+// split over CTAs matters.
+struct SensDep {
+    unsigned long long *acc;
+    uint32_t *h;
+    uint32_t n_g;
+    __device__ __forceinline__ SensDep(unsigned long long *smem, uint32_t n) : acc(smem), n_g(n) {
+        h = reinterpret_cast<uint32_t *>(smem + n);
+        for (uint32_t k = threadIdx.x; k < n_g; k += blockDim.x) {
+            acc[k] = 0ull;
+            h[k] = 0u;
+        }
+        __syncthreads();
+    }
+    // before round r of the CTA (every thread calls it)
+    __device__ __forceinline__ void round(uint32_t r) {
+        if (r == 0 || r % SENS_DEP_EPOCH != 0) return;
+        __syncthreads();
+        dep_drain(h, 1, n_g, acc, n_g);
+        __syncthreads();
+    }
+    __device__ __forceinline__ void flush(unsigned long long *hist) {
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < n_g; k += blockDim.x) {
+            const unsigned long long v = acc[k] + h[k];
+            if (v) atomicAdd(&hist[k], v);
+        }
+    }
+};
+size_t dep_smem(uint32_t n_g) { return (size_t)n_g * (sizeof(unsigned long long) + sizeof(uint32_t)); }
+
 __global__ void __launch_bounds__(SENS_THREADS)
     sens_deposit_kernel(const float *__restrict__ x, const uint32_t *__restrict__ n_ptr,
-                        unsigned long long *__restrict__ hist, const cudapic_grid g) {
-    extern __shared__ unsigned long long h[];
-    for (uint32_t k = threadIdx.x; k < g.n_g; k += blockDim.x) h[k] = 0ull;
-    __syncthreads();
+                        unsigned long long *__restrict__ hist, const __grid_constant__ cudapic_grid g) {
+    extern __shared__ unsigned long long sens_sm[];
+    SensDep dep(sens_sm, g.n_g);
+    grid_dep_wait();
     const uint32_t n = min(*n_ptr, g.capacity);
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        const float xv = x[p];
-        if (!(xv >= 0.0f)) continue;
-        const float pos = xv * g.inv_dx;
-        const int c = cell_of(pos, g.n_g);
-        const float rem = pos - (float)c;
-        const uint32_t r = min(__float2uint_rn(rem * (float)(1u << SENS_DEP_Q)), 1u << SENS_DEP_Q);
-        atomicAdd(&h[c], (unsigned long long)((1u << SENS_DEP_Q) - r));
-        atomicAdd(&h[c + 1], (unsigned long long)r);
+    const uint32_t stride = gridDim.x * blockDim.x;
+    uint32_t r = 0;
+    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x; b < n; b += stride, ++r) {
+        dep.round(r);
+        const uint64_t p = b + threadIdx.x;
+        if (p < n) {
+            const float xv = x[p];
+            if (xv >= 0.0f) dep_add(dep.h, xv, g);
+        }
     }
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < g.n_g; k += blockDim.x)
-        if (h[k]) atomicAdd(&hist[k], h[k]);
+    dep.flush(hist);
 }
 
-// Node sums -> f32 densities (boundary nodes doubled); clears the sums.
-__global__ void sens_density_kernel(unsigned long long *__restrict__ hist_e, unsigned long long *__restrict__ hist_i,
-                                    float *__restrict__ dens_e, float *__restrict__ dens_i, int ions,
-                                    const cudapic_grid g) {
-    const double w = g.weight_factor_d * (1.0 / (double)(1u << SENS_DEP_Q));
+// One more particle at x into the global node sums (a spawn).
+__device__ __forceinline__ void deposit_spawn(unsigned long long *hist, float x, const cudapic_grid &g) {
+    const float pos = x * g.inv_dx;
+    const int c = cell_of(pos, g.n_g);
+    const uint32_t r = min(__float2uint_rn((pos - (float)c) * (float)(1u << DEP_Q)), 1u << DEP_Q);
+    atomicAdd(&hist[c], (unsigned long long)((1u << DEP_Q) - r));
+    atomicAdd(&hist[c + 1], (unsigned long long)r);
+}
+
+// The field of a step, one CTA: marks the slot and record counts at the
+// step's start (mark may be null) and the spawn bases, turns the node sums
+// into f32 densities (boundary nodes doubled) and clears them, and solves
+// with the drivers' two-scan arithmetic (poisson_body), which the recompute
+// and the oracle's model repeat bit for bit.  efield: the step's field (on
+// the tape when recording).
+template <int PT>
+__global__ void __launch_bounds__(POIS_MAX_THREADS)
+    sens_field_kernel(uint32_t *__restrict__ cnt, uint32_t *__restrict__ mark, unsigned long long *__restrict__ hist_e,
+                      unsigned long long *__restrict__ hist_i, float *__restrict__ dens_e,
+                      float *__restrict__ dens_i, int ions, float *__restrict__ pot, float *__restrict__ efield,
+                      float pot0, const __grid_constant__ cudapic_grid g) {
+    grid_dep_wait();
+    if (threadIdx.x < 4 && mark) mark[threadIdx.x] = cnt[threadIdx.x];
+    if (threadIdx.x == 0) {
+        cnt[C_N0E] = min(cnt[C_NE], g.capacity);
+        cnt[C_N0I] = min(cnt[C_NI], g.capacity);
+    }
+    const double w = g.weight_factor_d * (1.0 / (double)(1u << DEP_Q));
     for (int s = 0; s < (ions ? 2 : 1); ++s) {
         unsigned long long *h = s ? hist_i : hist_e;
         float *d = s ? dens_i : dens_e;
@@ -295,17 +366,21 @@ __global__ void sens_density_kernel(unsigned long long *__restrict__ hist_e, uns
             h[k] = 0ull;
         }
     }
+    __syncthreads();
+    poisson_body<double, PT>(dens_e, dens_i, pot, efield, pot0, nullptr, nullptr, g, nullptr, nullptr);
 }
 
-// Push of the live slots in place (Rust-CUDA/src/main.rs:596-620); a particle
-// leaving [0, L] is marked dead.  obs (may be null) += the observable sum of
-// the species; tx / tv (may be null): the tape of x and v before the push.
+// Push of the live ions in place (Rust-CUDA/src/main.rs:596-620); a particle
+// leaving [0, L] is marked dead.  obs (may be null) += the observable sum;
+// tx / tv (may be null): the tape of x and v before the push.
 __global__ void __launch_bounds__(SENS_THREADS)
-    sens_push_kernel(float *__restrict__ x, float *__restrict__ vx, const uint32_t *__restrict__ n_ptr,
-                     const float *__restrict__ E, float f, float dt, int ions, double *__restrict__ obs,
-                     float *__restrict__ tx, float *__restrict__ tv, const cudapic_grid g) {
+    sens_push_i_kernel(float *__restrict__ x, float *__restrict__ vx, const uint32_t *__restrict__ n_ptr,
+                       const float *__restrict__ E, double *__restrict__ obs, float *__restrict__ tx,
+                       float *__restrict__ tv, const __grid_constant__ cudapic_grid g) {
     __shared__ double red[SENS_THREADS / 32];
+    grid_dep_wait();
     const uint32_t n = min(*n_ptr, g.capacity);
+    const float f = g.factor_i, dt = g.dt_i;
     double acc = 0.0;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const float xv = x[p], v = vx[p];
@@ -318,8 +393,7 @@ __global__ void __launch_bounds__(SENS_THREADS)
         const int c = cell_of(pos, g.n_g);
         const float c2 = pos - (float)c;
         const float ex = (1.0f - c2) * E[c] + c2 * E[c + 1];
-        if (!ions) acc += ((double)v + 0.5 * (double)f * (double)ex) * (double)ex;
-        else if (c == (int)g.n_g - 2) acc += (double)v * (double)c2;
+        if (c == (int)g.n_g - 2) acc += (double)v * (double)c2;
         const float v1 = v + f * ex;
         const float x1 = xv + v1 * dt;
         vx[p] = v1;
@@ -331,83 +405,130 @@ __global__ void __launch_bounds__(SENS_THREADS)
     }
 }
 
-// check_collisions_e (Rust-CUDA/src/main.rs:971-1033) over the slots live
-// before this step's spawns; an ionizing slot leaves its spawn request
+// The electrons of a step in one pass over the slots live before its spawns:
+// push (:596-620; tape, observable sum and dead marks as for the ions),
+// check_collisions_e (Rust-CUDA/src/main.rs:971-1033; the certain-rejection
+// bound of step.cuh first, the same decisions) and the deposit of the new
+// positions for the next step.  An ionizing slot leaves its spawn request
 // (children's velocities, record index) for the ranked spawn write.
 __global__ void __launch_bounds__(SENS_THREADS)
-    sens_collide_e_kernel(Planes e, uint32_t *__restrict__ cnt, const float *__restrict__ sig_e,
-                          const float *__restrict__ cs, SensRecE *__restrict__ rec, uint32_t rec_cap,
-                          uint32_t *__restrict__ spawn_rec, float *__restrict__ spawn_v,
-                          uint32_t *__restrict__ chunk_count, const cudapic_grid g) {
-    const uint32_t n = min(cnt[C_NE], g.capacity);
+    sens_electrons_kernel(Planes e, uint32_t *__restrict__ cnt, const float *__restrict__ E, double *__restrict__ obs,
+                          float *__restrict__ tx, float *__restrict__ tv, unsigned long long *__restrict__ hist,
+                          const float *__restrict__ sig_e, float sigma_max, const float *__restrict__ cs,
+                          SensRecE *__restrict__ rec, uint32_t rec_cap, uint32_t *__restrict__ spawn_rec,
+                          float *__restrict__ spawn_v, uint32_t *__restrict__ chunk_count,
+                          const __grid_constant__ cudapic_grid g) {
+    extern __shared__ unsigned long long sens_sm[];
+    __shared__ double red[SENS_THREADS / 32];
+    SensDep dep(sens_sm, g.n_g);
+    grid_dep_wait();
+    const uint32_t n = min(cnt[C_N0E], g.capacity);
     const uint32_t cap = g.capacity;
     const ScatK k{g.f1, g.f2};
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        if (!(e.x[p] >= 0.0f)) continue;
+    const float f = g.factor_e, dt = g.dt_e;
+    const float rej_k2 = sigma_max * dt * (sigma_max * dt) * 1.0001f;  // may_collide's bound
+    double acc = 0.0;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    uint32_t r = 0;
+    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x; b < n; b += stride, ++r) {
+        dep.round(r);
+        const uint32_t p = (uint32_t)b + threadIdx.x;
+        if (p >= n) continue;
+        const float xv = e.x[p], vo = e.vx[p];
+        if (tx) {
+            tx[p] = xv;
+            tv[p] = vo;
+        }
+        if (!(xv >= 0.0f)) continue;
+        const float vyp = e.vy[p], vzp = e.vz[p];
         Xoshiro128p rs{e.r[0][p], e.r[1][p], e.r[2][p], e.r[3][p]};
-        const float v[3] = {e.vx[p], e.vy[p], e.vz[p]};
-        const Test ts = test_electron(v[0], v[1], v[2], rs, GlobalTable{sig_e}, g);
-        if (ts.collide) {
-            const uint32_t idx = ts.idx;
-            const float t0 = __ldg(cs + idx);
-            const float t1 = t0 + __ldg(cs + CS_RANGES + idx);
-            const float t2 = t1 + __ldg(cs + 2 * CS_RANGES + idx);
-            const float rnd = rs.uniform();
-            int ev;
-            float a;
-            if (rnd < t0 / t2) {
-                ev = 1;
-                a = 1.0f - 2.0f * rs.uniform();
-            } else if (rnd < t1 / t2) {
-                ev = 2;
-                a = 1.0f - 2.0f * rs.uniform();
-            } else {
-                ev = 3;
-                a = rs.uniform();
-            }
-            const float eta = TWO_PI_F * rs.uniform();
-            float out[3], child[3];
-            scatter_e_t<float>(k, v, ev, a, eta, out, child);
-            uint32_t ri = SPAWN_NOREC;
-            if (rec) {
-                ri = atomicAdd(&cnt[C_REC_E], 1u);
-                if (ri < rec_cap) {
-                    SensRecE r;
-                    r.p = p;
-                    r.ev = (uint32_t)ev;
-                    r.ce = NO_SLOT;
-                    r.ci = NO_SLOT;
-                    r.v[0] = v[0];
-                    r.v[1] = v[1];
-                    r.v[2] = v[2];
-                    r.a = a;
-                    r.eta = eta;
-                    rec[ri] = r;
-                } else {
-                    set_dev_err(&cnt[C_ERR], CUDAPIC_DEVERR_RECORDS);
-                    ri = SPAWN_NOREC;
+        const float pos = xv * g.inv_dx;
+        const int c = cell_of(pos, g.n_g);
+        const float c2 = pos - (float)c;
+        const float ex = (1.0f - c2) * E[c] + c2 * E[c + 1];
+        acc += ((double)vo + 0.5 * (double)f * (double)ex) * (double)ex;
+        const float v1 = vo + f * ex;
+        const float x1 = xv + v1 * dt;
+        const bool stays = x1 >= 0.0f && x1 <= g.gap;
+        e.x[p] = stays ? x1 : -1.0f;
+        float vxn = v1;
+        if (stays) {
+            dep_add(dep.h, x1, g);
+            const float v[3] = {v1, vyp, vzp};
+            // test_electron's draw and decision
+            const float v2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+            const float u = rs.uniform();
+            if (may_collide(u, v2, rej_k2)) {
+                const uint32_t idx = energy_index(g.half_me_over_e * v2);
+                const float velocity = sqrtf(v2);
+                if (collision_draw(u, __ldg(sig_e + idx) * velocity * dt)) {
+                    const float t0 = __ldg(cs + idx);
+                    const float t1 = t0 + __ldg(cs + CS_RANGES + idx);
+                    const float t2 = t1 + __ldg(cs + 2 * CS_RANGES + idx);
+                    const float rnd = rs.uniform();
+                    int ev;
+                    float a;
+                    if (rnd < t0 / t2) {
+                        ev = 1;
+                        a = 1.0f - 2.0f * rs.uniform();
+                    } else if (rnd < t1 / t2) {
+                        ev = 2;
+                        a = 1.0f - 2.0f * rs.uniform();
+                    } else {
+                        ev = 3;
+                        a = rs.uniform();
+                    }
+                    const float eta = TWO_PI_F * rs.uniform();
+                    float out[3], child[3];
+                    scatter_e_t<float>(k, v, ev, a, eta, out, child);
+                    uint32_t ri = SPAWN_NOREC;
+                    if (rec) {
+                        ri = atomicAdd(&cnt[C_REC_E], 1u);
+                        if (ri < rec_cap) {
+                            SensRecE q;
+                            q.p = p;
+                            q.ev = (uint32_t)ev;
+                            q.ce = NO_SLOT;
+                            q.ci = NO_SLOT;
+                            q.v[0] = v[0];
+                            q.v[1] = v[1];
+                            q.v[2] = v[2];
+                            q.a = a;
+                            q.eta = eta;
+                            rec[ri] = q;
+                        } else {
+                            set_dev_err(&cnt[C_ERR], CUDAPIC_DEVERR_RECORDS);
+                            ri = SPAWN_NOREC;
+                        }
+                    }
+                    if (ev == 3) {
+                        float ia, ib, ic;
+                        rs.three_normal(g.normal_range, ia, ib, ic);
+                        spawn_v[0 * (size_t)cap + p] = child[0];
+                        spawn_v[1 * (size_t)cap + p] = child[1];
+                        spawn_v[2 * (size_t)cap + p] = child[2];
+                        spawn_v[3 * (size_t)cap + p] = ia;
+                        spawn_v[4 * (size_t)cap + p] = ib;
+                        spawn_v[5 * (size_t)cap + p] = ic;
+                        spawn_rec[p] = ri;
+                        atomicAdd(&chunk_count[p / SENS_CHUNK], 1u);
+                    }
+                    vxn = out[0];
+                    e.vy[p] = out[1];
+                    e.vz[p] = out[2];
                 }
             }
-            if (ev == 3) {
-                float ia, ib, ic;
-                rs.three_normal(g.normal_range, ia, ib, ic);
-                spawn_v[0 * (size_t)cap + p] = child[0];
-                spawn_v[1 * (size_t)cap + p] = child[1];
-                spawn_v[2 * (size_t)cap + p] = child[2];
-                spawn_v[3 * (size_t)cap + p] = ia;
-                spawn_v[4 * (size_t)cap + p] = ib;
-                spawn_v[5 * (size_t)cap + p] = ic;
-                spawn_rec[p] = ri;
-                atomicAdd(&chunk_count[p / SENS_CHUNK], 1u);
-            }
-            e.vx[p] = out[0];
-            e.vy[p] = out[1];
-            e.vz[p] = out[2];
+            e.r[0][p] = rs.s0;
+            e.r[1][p] = rs.s1;
+            e.r[2][p] = rs.s2;
+            e.r[3][p] = rs.s3;
         }
-        e.r[0][p] = rs.s0;
-        e.r[1][p] = rs.s1;
-        e.r[2][p] = rs.s2;
-        e.r[3][p] = rs.s3;
+        e.vx[p] = vxn;
+    }
+    dep.flush(hist);
+    if (obs) {
+        const double s = block_sum(acc, red);
+        if (threadIdx.x == 0 && s != 0.0) atomicAdd(obs, s);
     }
 }
 
@@ -435,56 +556,53 @@ __device__ __forceinline__ uint32_t block_excl_scan_u32(uint32_t v, uint32_t *ws
     return excl;
 }
 
-// One CTA: exclusive scan of the spawn counts of the chunks in slot order;
-// advances both counts (capped at the capacity, flagging dropped spawns).
-__global__ void __launch_bounds__(1024)
-    sens_spawn_scan_kernel(uint32_t *__restrict__ cnt, uint32_t *__restrict__ chunk_count,
-                           uint32_t *__restrict__ chunk_off, uint32_t cap) {
-    __shared__ uint32_t wsum[32];
-    const uint32_t n0e = min(cnt[C_NE], cap), n0i = min(cnt[C_NI], cap);
-    const uint32_t nch = (n0e + SENS_CHUNK - 1) / SENS_CHUNK;
-    uint32_t running = 0;
-    for (uint32_t base = 0; base < nch; base += blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const uint32_t v = i < nch ? chunk_count[i] : 0u;
-        uint32_t total;
-        const uint32_t ex = block_excl_scan_u32(v, wsum, total);
-        if (i < nch) {
-            chunk_off[i] = running + ex;
-            chunk_count[i] = 0u;
-        }
-        running += total;
-    }
-    if (threadIdx.x == 0) {
-        chunk_off[nch] = running;
-        cnt[C_N0E] = n0e;
-        cnt[C_N0I] = n0i;
-        const uint64_t ne = (uint64_t)n0e + running, ni = (uint64_t)n0i + running;
-        if (ne > cap) set_dev_err(&cnt[C_ERR], CUDAPIC_DEVERR_SPAWN_E);
-        if (ni > cap) set_dev_err(&cnt[C_ERR], CUDAPIC_DEVERR_SPAWN_I);
-        cnt[C_NE] = ne > cap ? cap : (uint32_t)ne;
-        cnt[C_NI] = ni > cap ? cap : (uint32_t)ni;
-    }
-}
-
-// One CTA of SENS_CHUNK threads per chunk with spawns: children at
-// n0 + chunk offset + rank of the parent among the chunk's spawning slots.
+// The spawns of a step in slot order, one CTA of SENS_CHUNK threads per chunk
+// with spawns: children at n0 + (spawns of the chunks before) + rank of the
+// parent among the chunk's spawning slots, the electron also added to the
+// next step's node sums.  Each such CTA sums the counts before its chunk
+// itself (spawns are rare: most CTAs read one count and leave), CTA 0 the
+// total, with which it advances both counts (capped at the capacity, dropped
+// spawns flagged).  `done`: the previous step's counts, cleared for the next.
 __global__ void __launch_bounds__(SENS_CHUNK)
-    sens_spawn_write_kernel(Planes e, Planes ion, const uint32_t *__restrict__ cnt,
-                            const uint32_t *__restrict__ chunk_off, uint32_t *__restrict__ spawn_rec,
-                            const float *__restrict__ spawn_v, SensRecE *__restrict__ rec, uint32_t cap) {
+    sens_spawn_kernel(Planes e, Planes ion, uint32_t *__restrict__ cnt, const uint32_t *__restrict__ chunk_count,
+                      uint32_t *__restrict__ done, uint32_t *__restrict__ spawn_rec,
+                      const float *__restrict__ spawn_v, SensRecE *__restrict__ rec,
+                      unsigned long long *__restrict__ hist_e, const __grid_constant__ cudapic_grid g) {
     __shared__ uint32_t wsum[32];
+    __shared__ uint32_t s_before;
+    grid_dep_wait();
+    const uint32_t cap = g.capacity;
     const uint32_t n0e = cnt[C_N0E], n0i = cnt[C_N0I];
     const uint32_t nch = (n0e + SENS_CHUNK - 1) / SENS_CHUNK;
+    if (blockIdx.x == 0) {
+        uint32_t sum = 0;
+        for (uint32_t k = threadIdx.x; k < nch; k += blockDim.x) sum += chunk_count[k];
+        uint32_t total;
+        block_excl_scan_u32(sum, wsum, total);
+        if (threadIdx.x == 0) {
+            const uint64_t ne = (uint64_t)n0e + total, ni = (uint64_t)n0i + total;
+            if (ne > cap) set_dev_err(&cnt[C_ERR], CUDAPIC_DEVERR_SPAWN_E);
+            if (ni > cap) set_dev_err(&cnt[C_ERR], CUDAPIC_DEVERR_SPAWN_I);
+            cnt[C_NE] = ne > cap ? cap : (uint32_t)ne;
+            cnt[C_NI] = ni > cap ? cap : (uint32_t)ni;
+        }
+    }
     for (uint32_t c = blockIdx.x; c < nch; c += gridDim.x) {
-        if (chunk_off[c + 1] == chunk_off[c]) continue;  // uniform in the block
+        if (threadIdx.x == 0) done[c] = 0u;
+        if (chunk_count[c] == 0) continue;  // uniform in the block
+        uint32_t sum = 0;
+        for (uint32_t k = threadIdx.x; k < c; k += blockDim.x) sum += chunk_count[k];
+        uint32_t before;
+        block_excl_scan_u32(sum, wsum, before);
+        if (threadIdx.x == 0) s_before = before;
+        __syncthreads();
         const uint32_t p = c * SENS_CHUNK + threadIdx.x;
         const uint32_t fl = p < n0e ? spawn_rec[p] : NO_SPAWN;
         const uint32_t flag = fl != NO_SPAWN ? 1u : 0u;
         uint32_t total;
         const uint32_t rank = block_excl_scan_u32(flag, wsum, total);
         if (flag) {
-            const uint32_t k = chunk_off[c] + rank;
+            const uint32_t k = s_before + rank;
             const uint32_t se = n0e + k, si = n0i + k;
             const float xp = e.x[p];
             uint32_t ce = NO_SLOT, ci = NO_SLOT;
@@ -493,6 +611,7 @@ __global__ void __launch_bounds__(SENS_CHUNK)
                 e.vx[se] = spawn_v[0 * (size_t)cap + p];
                 e.vy[se] = spawn_v[1 * (size_t)cap + p];
                 e.vz[se] = spawn_v[2 * (size_t)cap + p];
+                deposit_spawn(hist_e, xp, g);
                 ce = se;
             }
             if (si < cap) {
@@ -508,6 +627,7 @@ __global__ void __launch_bounds__(SENS_CHUNK)
             }
             spawn_rec[p] = NO_SPAWN;
         }
+        __syncthreads();  // s_before is rewritten for the next chunk
     }
 }
 
@@ -516,7 +636,8 @@ __global__ void __launch_bounds__(SENS_CHUNK)
 __global__ void __launch_bounds__(SENS_THREADS)
     sens_collide_i_kernel(Planes ion, uint32_t *__restrict__ cnt, const float *__restrict__ sig_i,
                           const float *__restrict__ cs, SensRecI *__restrict__ rec, uint32_t rec_cap,
-                          const cudapic_grid g) {
+                          const __grid_constant__ cudapic_grid g) {
+    grid_dep_wait();
     const uint32_t n = min(cnt[C_NI], g.capacity);
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         if (!(ion.x[p] >= 0.0f)) continue;
@@ -572,16 +693,30 @@ __global__ void sens_fill_kernel(float *__restrict__ p, uint32_t n, float v) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
 }
 
-// Tape mark of a step: slot counts and record counters at its start.
+// Tape mark of a segment's end: slot counts and record counters.
 __global__ void sens_mark_kernel(const uint32_t *__restrict__ cnt, uint32_t *__restrict__ mark) {
+    grid_dep_wait();
     if (threadIdx.x < 4) mark[threadIdx.x] = cnt[threadIdx.x];
 }
 
 // ------------------------------------------------------------------ adjoint
+// Both observables' adjoints go through the reverse sweep together (SENS_OBS
+// sets of planes): the tape, the records and the collision Jacobians are the
+// same for both.
+constexpr int SENS_OBS = 2;
+
+struct AdjPlanes {
+    float *x, *vx, *vy, *vz;
+};
+struct AdjSet {
+    AdjPlanes o[SENS_OBS];
+};
+
 __global__ void __launch_bounds__(SENS_THREADS)
     sens_adj_collide_i_kernel(const SensRecI *__restrict__ rec, const uint32_t *__restrict__ mark0,
-                              const uint32_t *__restrict__ mark1, uint32_t rec_cap, float *__restrict__ vbx,
-                              float *__restrict__ vby, float *__restrict__ vbz) {
+                              const uint32_t *__restrict__ mark1, uint32_t rec_cap,
+                              const __grid_constant__ AdjSet ion) {
+    grid_dep_wait();
     // an overflowed tape (flagged by the forward kernel) is read only up to its capacity
     const uint32_t b = min(mark0[C_REC_I], rec_cap), e = min(mark1[C_REC_I], rec_cap);
     for (uint32_t j = b + blockIdx.x * blockDim.x + threadIdx.x; j < e; j += gridDim.x * blockDim.x) {
@@ -589,102 +724,135 @@ __global__ void __launch_bounds__(SENS_THREADS)
         D3 v[3], out[3];
         for (int q = 0; q < 3; ++q) v[q] = seed(r.v[q], q);
         scatter_i_t<D3>(v, r.t, (int)r.ev, r.c, r.eta, out);
-        const float w[3] = {vbx[r.p], vby[r.p], vbz[r.p]};
-        float nv[3];
-        apply_jt(out, w, nv);
-        vbx[r.p] = nv[0];
-        vby[r.p] = nv[1];
-        vbz[r.p] = nv[2];
+#pragma unroll
+        for (int o = 0; o < SENS_OBS; ++o) {
+            const AdjPlanes &a = ion.o[o];
+            const float w[3] = {a.vx[r.p], a.vy[r.p], a.vz[r.p]};
+            float nv[3];
+            apply_jt(out, w, nv);
+            a.vx[r.p] = nv[0];
+            a.vy[r.p] = nv[1];
+            a.vz[r.p] = nv[2];
+        }
     }
 }
 
-struct AdjPlanes {
-    float *x, *vx, *vy, *vz;
-};
-
 __global__ void __launch_bounds__(SENS_THREADS)
     sens_adj_collide_e_kernel(const SensRecE *__restrict__ rec, const uint32_t *__restrict__ mark0,
-                              const uint32_t *__restrict__ mark1, uint32_t rec_cap, AdjPlanes e, AdjPlanes ion,
-                              const cudapic_grid g) {
+                              const uint32_t *__restrict__ mark1, uint32_t rec_cap, const __grid_constant__ AdjSet es,
+                              const __grid_constant__ AdjSet is, const __grid_constant__ cudapic_grid g) {
+    grid_dep_wait();
     const uint32_t b = min(mark0[C_REC_E], rec_cap), en = min(mark1[C_REC_E], rec_cap);
     const ScatK k{g.f1, g.f2};
     for (uint32_t j = b + blockIdx.x * blockDim.x + threadIdx.x; j < en; j += gridDim.x * blockDim.x) {
         const SensRecE r = rec[j];
+        const uint32_t p = r.p;
+        // the adjoints gathered before the Jacobian is formed: their latency hides behind it
+        float w[SENS_OBS][3], xb[SENS_OBS];
+#pragma unroll
+        for (int o = 0; o < SENS_OBS; ++o) {
+            w[o][0] = es.o[o].vx[p];
+            w[o][1] = es.o[o].vy[p];
+            w[o][2] = es.o[o].vz[p];
+            xb[o] = es.o[o].x[p];
+        }
         D3 v[3], out[3], child[3];
         for (int q = 0; q < 3; ++q) v[q] = seed(r.v[q], q);
         scatter_e_t<D3>(k, v, (int)r.ev, r.a, r.eta, out, child);
-        const uint32_t p = r.p;
-        const float w[3] = {e.vx[p], e.vy[p], e.vz[p]};
-        float nv[3];
-        apply_jt(out, w, nv);
-        float xb = e.x[p];
-        if (r.ev == 3 && r.ce != NO_SLOT) {
-            const uint32_t s = r.ce;
-            const float wc[3] = {e.vx[s], e.vy[s], e.vz[s]};
-            float nc[3];
-            apply_jt(child, wc, nc);
-            for (int q = 0; q < 3; ++q) nv[q] += nc[q];
-            xb += e.x[s];
-            e.x[s] = e.vx[s] = e.vy[s] = e.vz[s] = 0.0f;
+#pragma unroll
+        for (int o = 0; o < SENS_OBS; ++o) {
+            const AdjPlanes &e = es.o[o], &ion = is.o[o];
+            float nv[3];
+            apply_jt(out, w[o], nv);
+            if (r.ev == 3 && r.ce != NO_SLOT) {
+                const uint32_t s = r.ce;
+                const float wc[3] = {e.vx[s], e.vy[s], e.vz[s]};
+                float nc[3];
+                apply_jt(child, wc, nc);
+                for (int q = 0; q < 3; ++q) nv[q] += nc[q];
+                xb[o] += e.x[s];
+                e.x[s] = e.vx[s] = e.vy[s] = e.vz[s] = 0.0f;
+            }
+            if (r.ev == 3 && r.ci != NO_SLOT) {
+                const uint32_t s = r.ci;
+                xb[o] += ion.x[s];
+                ion.x[s] = ion.vx[s] = ion.vy[s] = ion.vz[s] = 0.0f;
+            }
+            e.x[p] = xb[o];
+            e.vx[p] = nv[0];
+            e.vy[p] = nv[1];
+            e.vz[p] = nv[2];
         }
-        if (r.ev == 3 && r.ci != NO_SLOT) {
-            const uint32_t s = r.ci;
-            xb += ion.x[s];
-            ion.x[s] = ion.vx[s] = ion.vy[s] = ion.vz[s] = 0.0f;
-        }
-        e.x[p] = xb;
-        e.vx[p] = nv[0];
-        e.vy[p] = nv[1];
-        e.vz[p] = nv[2];
     }
 }
 
-// Adjoint of the push (and of the species' observable term, weight wo) of
-// the slots live at the step's start; the field adjoint is summed in FP64.
+// Adjoint of the push (and of the species' observable term, weight wo[o] for
+// observable o) of the slots live at the step's start; the field adjoints
+// (eb: [SENS_OBS][n_g]) are summed in FP64.
+struct ObsWeights {
+    float w[SENS_OBS];
+};
+
 __global__ void __launch_bounds__(SENS_THREADS)
     sens_adj_push_kernel(const float *__restrict__ tx, const float *__restrict__ tv, const uint32_t *__restrict__ n_ptr,
-                         const float *__restrict__ E, float f, float dt, int ions, float wo, float *__restrict__ xb,
-                         float *__restrict__ vb, double *__restrict__ eb, const cudapic_grid g) {
-    extern __shared__ double ebs[];
-    for (uint32_t k = threadIdx.x; k < g.n_g; k += blockDim.x) ebs[k] = 0.0;
+                         const float *__restrict__ E, float f, float dt, int ions, const ObsWeights wo,
+                         const __grid_constant__ AdjSet adj, double *__restrict__ eb,
+                         const __grid_constant__ cudapic_grid g) {
+    extern __shared__ double ebs[];  // [SENS_OBS][n_g]
+    const uint32_t n_g = g.n_g;
+    for (uint32_t k = threadIdx.x; k < SENS_OBS * n_g; k += blockDim.x) ebs[k] = 0.0;
     __syncthreads();
+    grid_dep_wait();
     const uint32_t n = min(*n_ptr, g.capacity);
     const float inv_dx = g.inv_dx;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const float x = tx[p];
-        if (!(x >= 0.0f)) continue;
         const float v = tv[p];
+        float a[SENS_OBS], b[SENS_OBS];
+#pragma unroll
+        for (int o = 0; o < SENS_OBS; ++o) {
+            a[o] = adj.o[o].x[p];
+            b[o] = adj.o[o].vx[p];
+        }
+        if (!(x >= 0.0f)) continue;
         const float pos = x * inv_dx;
-        const int c = cell_of(pos, g.n_g);
+        const int c = cell_of(pos, n_g);
         const float c2 = pos - (float)c;
         const float e0 = E[c], e1 = E[c + 1];
         const float ex = (1.0f - c2) * e0 + c2 * e1;
         const float dex = (e1 - e0) * inv_dx;
-        const float a = xb[p], b = vb[p];
-        const float bt = b + dt * a;
-        float nx = a, nv = bt, eg = bt * f;
-        if (!ions) {
-            nv += wo * ex;
-            eg += wo * (v + f * ex);
-        } else if (c == (int)g.n_g - 2) {
-            nv += wo * c2;
-            nx += wo * v * inv_dx;
+#pragma unroll
+        for (int o = 0; o < SENS_OBS; ++o) {
+            const float bt = b[o] + dt * a[o];
+            float nx = a[o], nv = bt, eg = bt * f;
+            if (!ions) {
+                nv += wo.w[o] * ex;
+                eg += wo.w[o] * (v + f * ex);
+            } else if (c == (int)n_g - 2) {
+                nv += wo.w[o] * c2;
+                nx += wo.w[o] * v * inv_dx;
+            }
+            nx += eg * dex;
+            if (eg != 0.0f) {
+                atomicAdd(&ebs[o * n_g + c], (double)eg * (double)(1.0f - c2));
+                atomicAdd(&ebs[o * n_g + c + 1], (double)eg * (double)c2);
+            }
+            adj.o[o].x[p] = nx;
+            adj.o[o].vx[p] = nv;
         }
-        nx += eg * dex;
-        atomicAdd(&ebs[c], (double)eg * (double)(1.0f - c2));
-        atomicAdd(&ebs[c + 1], (double)eg * (double)c2);
-        xb[p] = nx;
-        vb[p] = nv;
     }
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < g.n_g; k += blockDim.x)
+    for (uint32_t k = threadIdx.x; k < SENS_OBS * n_g; k += blockDim.x)
         if (ebs[k] != 0.0) atomicAdd(&eb[k], ebs[k]);
 }
 
-// Deposit adjoint: x adjoint += d/dx sum_k db[k] n_k(x) (CIC, boundary nodes doubled).
+// Deposit adjoint: x adjoint += d/dx sum_k db[k] n_k(x) (CIC, boundary nodes
+// doubled); db: [SENS_OBS][n_g].
 __global__ void __launch_bounds__(SENS_THREADS)
     sens_adj_gather_kernel(const float *__restrict__ tx, const uint32_t *__restrict__ n_ptr,
-                           const double *__restrict__ db, float *__restrict__ xb, const cudapic_grid g) {
+                           const double *__restrict__ db, const __grid_constant__ AdjSet adj,
+                           const __grid_constant__ cudapic_grid g) {
+    grid_dep_wait();
     const uint32_t n = min(*n_ptr, g.capacity);
     const double k = g.weight_factor_d / g.dx;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
@@ -692,7 +860,11 @@ __global__ void __launch_bounds__(SENS_THREADS)
         if (!(x >= 0.0f)) continue;
         const int c = cell_of(x * g.inv_dx, g.n_g);
         const double b0 = c == 0 ? 2.0 : 1.0, b1 = (c + 1 == (int)g.n_g - 1) ? 2.0 : 1.0;
-        xb[p] += (float)(k * (b1 * db[c + 1] - b0 * db[c]));
+#pragma unroll
+        for (int o = 0; o < SENS_OBS; ++o) {
+            const double *d = db + (size_t)o * g.n_g;
+            adj.o[o].x[p] += (float)(k * (b1 * d[c + 1] - b0 * d[c]));
+        }
     }
 }
 
@@ -717,7 +889,8 @@ struct cudapic_sens {
     unsigned long long *hist = nullptr;  // [2][n_g]
     float *dens = nullptr, *efield = nullptr, *pot = nullptr;
     double *obs = nullptr;               // [2] raw sums
-    uint32_t *spawn_rec = nullptr, *chunk_count = nullptr, *chunk_off = nullptr;
+    uint32_t *spawn_rec = nullptr;
+    uint32_t *chunk_count[2] = {nullptr, nullptr};  // spawns per chunk, by the parity of the step
     float *spawn_v = nullptr;
     float *ckpt = nullptr;               // [n_seg][2][8][cap] (RNG planes stored bitwise)
     uint32_t *ckpt_cnt = nullptr;        // [n_seg][C_COUNT]
@@ -725,8 +898,8 @@ struct cudapic_sens {
     uint32_t *tmark = nullptr;           // [S + 1][4]
     SensRecE *rec_e = nullptr;
     SensRecI *rec_i = nullptr;
-    float *adj = nullptr;                // [2][4][cap]
-    double *eb = nullptr, *neb = nullptr, *nib_acc = nullptr, *vbar = nullptr;
+    float *adj = nullptr;                // [SENS_OBS][2][4][cap]
+    double *eb = nullptr, *neb = nullptr, *nib_acc = nullptr, *vbar = nullptr;  // [SENS_OBS][n_g], vbar [SENS_OBS]
     std::vector<void *> allocs;
     size_t bytes = 0;
 };
@@ -761,9 +934,13 @@ Planes planes_of(float *base, uint32_t cap) {
     return p;
 }
 
-AdjPlanes adj_of(const cudapic_sens *s, int sp) {
-    float *b = s->adj + (size_t)sp * 4 * s->cap;
-    return {b, b + s->cap, b + 2 * (size_t)s->cap, b + 3 * (size_t)s->cap};
+AdjSet adj_of(const cudapic_sens *s, int sp) {
+    AdjSet a;
+    for (int o = 0; o < SENS_OBS; ++o) {
+        float *b = s->adj + ((size_t)o * 2 + sp) * 4 * s->cap;
+        a.o[o] = {b, b + s->cap, b + 2 * (size_t)s->cap, b + 3 * (size_t)s->cap};
+    }
+    return a;
 }
 
 unsigned grid_n(uint32_t units) { return persistent_grid(SENS_PER_SM, (units + SENS_THREADS - 1) / SENS_THREADS); }
@@ -787,44 +964,52 @@ void obs_scale(const cudapic_sens *s, double *cP, double *cG) {
     *cG = 2.0 * s->g.weight_factor_d / (double)(k_i ? k_i : 1);
 }
 
+int launch_field(cudapic_sens *s, float *efield, uint32_t *mark, int ions, float pot0) {
+    int threads, pt;
+    poisson_shape(s->n_g, threads, pt);
+    auto kern = pt == 1 ? sens_field_kernel<1> : pt == 2 ? sens_field_kernel<2> : sens_field_kernel<4>;  // n_g <= 4096
+    return launch_kernel("sens_field", kern, 1, threads, sizeof(double) * s->n_g, s->stream, s->cnt, mark, s->hist,
+                         s->hist + s->n_g, s->dens, s->dens + s->n_g, ions, s->pot, efield, pot0, s->g);
+}
+
+// Before the first step of a run or segment: the node sums of its electrons,
+// no spawns counted.
+int start_steps(cudapic_sens *s) {
+    CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->hist, 0, sizeof(unsigned long long) * 2 * s->n_g, s->stream), "sens hist"));
+    for (auto *c : s->chunk_count)
+        CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(c, 0, sizeof(uint32_t) * (s->cap / SENS_CHUNK + 2), s->stream),
+                                 "sens chunks"));
+    return launch_kernel("sens_deposit", sens_deposit_kernel, grid_n(s->cap), SENS_THREADS, dep_smem(s->n_g), s->stream,
+                         s->cur[0].x, s->cnt + C_NE, s->hist, s->g);
+}
+
 // One forward step t; rec: record the tape at step j of the segment.
 int fwd_step(cudapic_sens *s, uint32_t t, bool rec, uint32_t j) {
     cudaStream_t st = s->stream;
     const cudapic_grid &g = s->g;
     const bool ions = ion_step(s, t);
     const size_t cap = s->cap;
-    if (rec) CUDAPIC_CHECK(launch_kernel("sens_mark", sens_mark_kernel, 1, 32, 0, st, s->cnt, s->tmark + 4 * j));
     const unsigned gd = grid_n(s->cap);
-    const size_t hsm = sizeof(unsigned long long) * s->n_g;
-    CUDAPIC_CHECK(launch_kernel("sens_deposit", sens_deposit_kernel, gd, SENS_THREADS, hsm, st, s->cur[0].x,
-                                s->cnt + C_NE, s->hist, g));
     if (ions)
-        CUDAPIC_CHECK(launch_kernel("sens_deposit", sens_deposit_kernel, gd, SENS_THREADS, hsm, st, s->cur[1].x,
-                                    s->cnt + C_NI, s->hist + s->n_g, g));
-    CUDAPIC_CHECK(launch_kernel("sens_density", sens_density_kernel, 1, 512, 0, st, s->hist, s->hist + s->n_g,
-                                s->dens, s->dens + s->n_g, ions ? 1 : 0, g));
-    CUDAPIC_CHECK(launch_poisson(s->dens, s->dens + s->n_g, s->pot, s->efield, pot0_at(s, t), nullptr, nullptr, g, st));
-    if (rec)
-        CUDAPIC_CHECK(check_cuda(cudaMemcpyAsync(s->tE + (size_t)j * s->n_g, s->efield, sizeof(float) * s->n_g,
-                                                 cudaMemcpyDeviceToDevice, st), "sensitivity field tape"));
-    CUDAPIC_CHECK(launch_kernel("sens_push", sens_push_kernel, gd, SENS_THREADS, 0, st, s->cur[0].x, s->cur[0].vx,
-                                s->cnt + C_NE, s->efield, g.factor_e, g.dt_e, 0, rec ? nullptr : s->obs,
-                                rec ? s->tx_e + j * cap : nullptr, rec ? s->tv_e + j * cap : nullptr, g));
+        CUDAPIC_CHECK(launch_kernel("sens_deposit", sens_deposit_kernel, gd, SENS_THREADS, dep_smem(s->n_g), st,
+                                    s->cur[1].x, s->cnt + C_NI, s->hist + s->n_g, g));
+    float *E = rec ? s->tE + (size_t)j * s->n_g : s->efield;
+    CUDAPIC_CHECK(launch_field(s, E, rec ? s->tmark + 4 * j : nullptr, ions ? 1 : 0, pot0_at(s, t)));
+    CUDAPIC_CHECK(launch_kernel("sens_electrons", sens_electrons_kernel, gd, SENS_THREADS, dep_smem(s->n_g), st,
+                                s->cur[0], s->cnt, E, rec ? nullptr : s->obs, rec ? s->tx_e + j * cap : nullptr,
+                                rec ? s->tv_e + j * cap : nullptr, s->hist, s->st->sigma_tot_e, s->st->sigma_max_e,
+                                s->st->cs, rec ? s->rec_e : nullptr, s->rec_cap_e, s->spawn_rec, s->spawn_v,
+                                s->chunk_count[t & 1u], g));
     if (ions) {
         const size_t ji = j / s->n_sub;
-        CUDAPIC_CHECK(launch_kernel("sens_push", sens_push_kernel, gd, SENS_THREADS, 0, st, s->cur[1].x, s->cur[1].vx,
-                                    s->cnt + C_NI, s->efield, g.factor_i, g.dt_i, 1, rec ? nullptr : s->obs + 1,
+        CUDAPIC_CHECK(launch_kernel("sens_push_i", sens_push_i_kernel, gd, SENS_THREADS, 0, st, s->cur[1].x,
+                                    s->cur[1].vx, s->cnt + C_NI, E, rec ? nullptr : s->obs + 1,
                                     rec ? s->tx_i + ji * cap : nullptr, rec ? s->tv_i + ji * cap : nullptr, g));
     }
-    CUDAPIC_CHECK(launch_kernel("sens_collide_e", sens_collide_e_kernel, gd, SENS_THREADS, 0, st, s->cur[0], s->cnt,
-                                s->st->sigma_tot_e, s->st->cs, rec ? s->rec_e : nullptr, s->rec_cap_e, s->spawn_rec,
-                                s->spawn_v, s->chunk_count, g));
-    CUDAPIC_CHECK(launch_kernel("sens_spawn_scan", sens_spawn_scan_kernel, 1, 1024, 0, st, s->cnt, s->chunk_count,
-                                s->chunk_off, s->cap));
     const unsigned nch = (s->cap + SENS_CHUNK - 1) / SENS_CHUNK;
-    CUDAPIC_CHECK(launch_kernel("sens_spawn_write", sens_spawn_write_kernel, std::min<unsigned>(nch, 4096u),
-                                SENS_CHUNK, 0, st, s->cur[0], s->cur[1], s->cnt, s->chunk_off, s->spawn_rec,
-                                s->spawn_v, rec ? s->rec_e : nullptr, s->cap));
+    CUDAPIC_CHECK(launch_kernel("sens_spawn", sens_spawn_kernel, std::min<unsigned>(nch, 4096u), SENS_CHUNK, 0, st,
+                                s->cur[0], s->cur[1], s->cnt, s->chunk_count[t & 1u], s->chunk_count[(t & 1u) ^ 1u],
+                                s->spawn_rec, s->spawn_v, rec ? s->rec_e : nullptr, s->hist, g));
     if (ions)
         CUDAPIC_CHECK(launch_kernel("sens_collide_i", sens_collide_i_kernel, gd, SENS_THREADS, 0, st, s->cur[1], s->cnt,
                                     s->st->sigma_tot_i, s->st->cs, rec ? s->rec_i : nullptr, s->rec_cap_i, g));
@@ -838,36 +1023,36 @@ int copy_planes(cudapic_sens *s, float *dst, const float *src) {
 }
 
 // Reverse step t (segment step j).
-int adj_step(cudapic_sens *s, uint32_t t, uint32_t j, float wP, float wG) {
+int adj_step(cudapic_sens *s, uint32_t t, uint32_t j, const ObsWeights &wP, const ObsWeights &wG) {
     cudaStream_t st = s->stream;
     const cudapic_grid &g = s->g;
     const bool ions = ion_step(s, t);
     const size_t cap = s->cap;
     const uint32_t *m0 = s->tmark + 4 * j, *m1 = s->tmark + 4 * (j + 1);
     const unsigned gd = grid_n(s->cap);
-    AdjPlanes ae = adj_of(s, 0), ai = adj_of(s, 1);
+    const AdjSet ae = adj_of(s, 0), ai = adj_of(s, 1);
     if (ions)
         CUDAPIC_CHECK(launch_kernel("sens_adj_collide_i", sens_adj_collide_i_kernel, gd, SENS_THREADS, 0, st, s->rec_i,
-                                    m0, m1, s->rec_cap_i, ai.vx, ai.vy, ai.vz));
+                                    m0, m1, s->rec_cap_i, ai));
     CUDAPIC_CHECK(launch_kernel("sens_adj_collide_e", sens_adj_collide_e_kernel, gd, SENS_THREADS, 0, st, s->rec_e, m0,
                                 m1, s->rec_cap_e, ae, ai, g));
     const float *E = s->tE + (size_t)j * s->n_g;
-    const size_t esm = sizeof(double) * s->n_g;
+    const size_t esm = sizeof(double) * SENS_OBS * s->n_g;
     CUDAPIC_CHECK(launch_kernel("sens_adj_push", sens_adj_push_kernel, gd, SENS_THREADS, esm, st, s->tx_e + j * cap,
-                                s->tv_e + j * cap, m0 + C_NE, E, g.factor_e, g.dt_e, 0, wP, ae.x, ae.vx, s->eb, g));
+                                s->tv_e + j * cap, m0 + C_NE, E, g.factor_e, g.dt_e, 0, wP, ae, s->eb, g));
     const size_t ji = j / s->n_sub;
     if (ions)
         CUDAPIC_CHECK(launch_kernel("sens_adj_push", sens_adj_push_kernel, gd, SENS_THREADS, esm, st,
                                     s->tx_i + ji * cap, s->tv_i + ji * cap, m0 + C_NI, E, g.factor_i, g.dt_i, 1, wG,
-                                    ai.x, ai.vx, s->eb, g));
+                                    ai, s->eb, g));
     // the ion-density adjoint gathered at step t + 1 (an ion step) restarts
     CUDAPIC_CHECK(launch_poisson_adjoint(s->eb, s->neb, s->nib_acc, ion_step(s, t + 1) ? 1 : 0, cos_at(s, t), s->vbar,
-                                         g, st));
+                                         SENS_OBS, g, st));
     CUDAPIC_CHECK(launch_kernel("sens_adj_gather", sens_adj_gather_kernel, gd, SENS_THREADS, 0, st, s->tx_e + j * cap,
-                                m0 + C_NE, (const double *)s->neb, ae.x, g));
+                                m0 + C_NE, (const double *)s->neb, ae, g));
     if (ions)
         CUDAPIC_CHECK(launch_kernel("sens_adj_gather", sens_adj_gather_kernel, gd, SENS_THREADS, 0, st,
-                                    s->tx_i + ji * cap, m0 + C_NI, (const double *)s->nib_acc, ai.x, g));
+                                    s->tx_i + ji * cap, m0 + C_NI, (const double *)s->nib_acc, ai, g));
     return CUDAPIC_OK;
 }
 
@@ -921,8 +1106,8 @@ extern "C" int cudapic_sens_create(cudapic_state *st, uint32_t window_steps, uin
         (rc = sens_alloc_t(s, &s->dens, 2 * (size_t)s->n_g)) || (rc = sens_alloc_t(s, &s->efield, s->n_g)) ||
         (rc = sens_alloc_t(s, &s->pot, s->n_g)) || (rc = sens_alloc_t(s, &s->obs, 2)) ||
         (rc = sens_alloc_t(s, &s->spawn_rec, cap)) || (rc = sens_alloc_t(s, &s->spawn_v, 6 * cap)) ||
-        (rc = sens_alloc_t(s, &s->chunk_count, cap / SENS_CHUNK + 2)) ||
-        (rc = sens_alloc_t(s, &s->chunk_off, cap / SENS_CHUNK + 2)) ||
+        (rc = sens_alloc_t(s, &s->chunk_count[0], cap / SENS_CHUNK + 2)) ||
+        (rc = sens_alloc_t(s, &s->chunk_count[1], cap / SENS_CHUNK + 2)) ||
         (rc = sens_alloc_t(s, &s->ckpt, (size_t)s->n_seg * 16 * cap)) ||
         (rc = sens_alloc_t(s, &s->ckpt_cnt, (size_t)s->n_seg * C_COUNT)) ||
         (rc = sens_alloc_t(s, &s->tx_e, (size_t)s->S * cap)) || (rc = sens_alloc_t(s, &s->tv_e, (size_t)s->S * cap)) ||
@@ -931,9 +1116,18 @@ extern "C" int cudapic_sens_create(cudapic_state *st, uint32_t window_steps, uin
         (rc = sens_alloc_t(s, &s->tE, (size_t)s->S * s->n_g)) ||
         (rc = sens_alloc_t(s, &s->tmark, 4 * ((size_t)s->S + 1))) ||
         (rc = sens_alloc_t(s, &s->rec_e, s->rec_cap_e)) || (rc = sens_alloc_t(s, &s->rec_i, s->rec_cap_i)) ||
-        (rc = sens_alloc_t(s, &s->adj, 8 * cap)) || (rc = sens_alloc_t(s, &s->eb, s->n_g)) ||
-        (rc = sens_alloc_t(s, &s->neb, s->n_g)) || (rc = sens_alloc_t(s, &s->nib_acc, s->n_g)) ||
-        (rc = sens_alloc_t(s, &s->vbar, 1)))
+        (rc = sens_alloc_t(s, &s->adj, SENS_OBS * 8 * cap)) || (rc = sens_alloc_t(s, &s->eb, SENS_OBS * (size_t)s->n_g)) ||
+        (rc = sens_alloc_t(s, &s->neb, SENS_OBS * (size_t)s->n_g)) ||
+        (rc = sens_alloc_t(s, &s->nib_acc, SENS_OBS * (size_t)s->n_g)) || (rc = sens_alloc_t(s, &s->vbar, SENS_OBS)))
+        return fail_free(rc);
+    // above the 48 KB a launch may take by default (n_g up to 4096)
+    if ((rc = check_cuda(cudaFuncSetAttribute(sens_deposit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)dep_smem(SENS_MAX_NG)), "cudaFuncSetAttribute(sens)")) ||
+        (rc = check_cuda(cudaFuncSetAttribute(sens_electrons_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)dep_smem(SENS_MAX_NG)), "cudaFuncSetAttribute(sens)")) ||
+        (rc = check_cuda(cudaFuncSetAttribute(sens_adj_push_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)(sizeof(double) * SENS_OBS * SENS_MAX_NG)),
+                         "cudaFuncSetAttribute(sens)")))
         return fail_free(rc);
     for (int sp = 0; sp < 2; ++sp) {
         s->init[sp] = planes_of(init + (size_t)sp * 8 * cap, s->cap);
@@ -969,8 +1163,6 @@ extern "C" int cudapic_sens_create(cudapic_state *st, uint32_t window_steps, uin
         }
     }
     if ((rc = check_cuda(cudaMemsetAsync(s->spawn_rec, 0xFF, sizeof(uint32_t) * cap, sm), "sens spawn flags")) ||
-        (rc = check_cuda(cudaMemsetAsync(s->chunk_count, 0, sizeof(uint32_t) * (cap / SENS_CHUNK + 2), sm), "sens chunks")) ||
-        (rc = check_cuda(cudaMemsetAsync(s->hist, 0, sizeof(unsigned long long) * 2 * s->n_g, sm), "sens hist")) ||
         (rc = check_cuda(cudaStreamSynchronize(sm), "sens create sync")))
         return fail_free(rc);
     *out = s;
@@ -989,6 +1181,8 @@ extern "C" int cudapic_sens_forward(cudapic_sens *s, double voltage, double obs[
     uint32_t c0[C_COUNT] = {s->n_init[0], s->n_init[1], 0, 0, 0, 0, 0, 0};
     CUDAPIC_CHECK(check_cuda(cudaMemcpyAsync(s->cnt, c0, sizeof(c0), cudaMemcpyHostToDevice, st), "sens counters"));
     CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->obs, 0, 2 * sizeof(double), st), "sens obs"));
+    PdlScope pdl(true);
+    CUDAPIC_CHECK(start_steps(s));
     for (uint32_t t = 0; t < s->K; ++t) {
         if (t % s->S == 0) {
             const uint32_t k = t / s->S;
@@ -1019,33 +1213,34 @@ extern "C" int cudapic_sens_backward(cudapic_sens *s, double grad[2]) {
     const size_t cap = s->cap;
     double cP, cG;
     obs_scale(s, &cP, &cG);
-    for (int o = 0; o < 2; ++o) {
-        const float wP = o == 0 ? (float)cP : 0.0f, wG = o == 1 ? (float)cG : 0.0f;
-        CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->adj, 0, sizeof(float) * 8 * cap, st), "sens adjoint"));
-        CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->eb, 0, sizeof(double) * s->n_g, st), "sens eb"));
-        CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->nib_acc, 0, sizeof(double) * s->n_g, st), "sens nib"));
-        CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->vbar, 0, sizeof(double), st), "sens vbar"));
-        for (int64_t k = (int64_t)s->n_seg - 1; k >= 0; --k) {
-            const uint32_t t0 = (uint32_t)k * s->S;
-            if (s->H && (t0 + s->S) % s->H == 0)  // a horizon ends after this segment: the adjoint restarts
-                CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->adj, 0, sizeof(float) * 8 * cap, st), "sens horizon"));
-            // recompute the segment from its checkpoint, recording the tape
-            CUDAPIC_CHECK(copy_planes(s, s->cur[0].x, s->ckpt + (size_t)k * 16 * cap));
-            CUDAPIC_CHECK(check_cuda(cudaMemcpyAsync(s->cnt, s->ckpt_cnt + (size_t)k * C_COUNT, sizeof(uint32_t) * C_COUNT,
-                                                     cudaMemcpyDeviceToDevice, st), "sens restore counters"));
-            CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->cnt + C_REC_E, 0, 2 * sizeof(uint32_t), st), "sens records"));
-            for (uint32_t j = 0; j < s->S; ++j) CUDAPIC_CHECK(fwd_step(s, t0 + j, true, j));
-            CUDAPIC_CHECK(launch_kernel("sens_mark", sens_mark_kernel, 1, 32, 0, st, s->cnt, s->tmark + 4 * s->S));
-            for (int64_t j = (int64_t)s->S - 1; j >= 0; --j)
-                CUDAPIC_CHECK(adj_step(s, t0 + (uint32_t)j, (uint32_t)j, wP, wG));
-        }
-        CUDAPIC_CHECK(check_cuda(cudaMemcpyAsync(&grad[o], s->vbar, sizeof(double), cudaMemcpyDeviceToHost, st),
-                                 "sens gradient read"));
-        uint32_t err = 0;
-        CUDAPIC_CHECK(read_err(s, &err));
-        if (err & CUDAPIC_DEVERR_RECORDS) return fail(CUDAPIC_ERR_CAPACITY, "sens_backward: collision records overflowed");
-        if (err) return fail(CUDAPIC_ERR_CAPACITY, "sens_backward: device error (spawns beyond the capacity)");
+    const ObsWeights wP{{(float)cP, 0.0f}}, wG{{0.0f, (float)cG}};
+    const size_t adj_bytes = sizeof(float) * SENS_OBS * 8 * cap, node_bytes = sizeof(double) * SENS_OBS * s->n_g;
+    CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->adj, 0, adj_bytes, st), "sens adjoint"));
+    CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->eb, 0, node_bytes, st), "sens eb"));
+    CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->nib_acc, 0, node_bytes, st), "sens nib"));
+    CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->vbar, 0, SENS_OBS * sizeof(double), st), "sens vbar"));
+    PdlScope pdl(true);
+    for (int64_t k = (int64_t)s->n_seg - 1; k >= 0; --k) {
+        const uint32_t t0 = (uint32_t)k * s->S;
+        if (s->H && (t0 + s->S) % s->H == 0)  // a horizon ends after this segment: the adjoint restarts
+            CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->adj, 0, adj_bytes, st), "sens horizon"));
+        // recompute the segment from its checkpoint, recording the tape
+        CUDAPIC_CHECK(copy_planes(s, s->cur[0].x, s->ckpt + (size_t)k * 16 * cap));
+        CUDAPIC_CHECK(check_cuda(cudaMemcpyAsync(s->cnt, s->ckpt_cnt + (size_t)k * C_COUNT, sizeof(uint32_t) * C_COUNT,
+                                                 cudaMemcpyDeviceToDevice, st), "sens restore counters"));
+        CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->cnt + C_REC_E, 0, 2 * sizeof(uint32_t), st), "sens records"));
+        CUDAPIC_CHECK(start_steps(s));
+        for (uint32_t j = 0; j < s->S; ++j) CUDAPIC_CHECK(fwd_step(s, t0 + j, true, j));
+        CUDAPIC_CHECK(launch_kernel("sens_mark", sens_mark_kernel, 1, 32, 0, st, s->cnt, s->tmark + 4 * s->S));
+        for (int64_t j = (int64_t)s->S - 1; j >= 0; --j)
+            CUDAPIC_CHECK(adj_step(s, t0 + (uint32_t)j, (uint32_t)j, wP, wG));
     }
+    CUDAPIC_CHECK(check_cuda(cudaMemcpyAsync(grad, s->vbar, SENS_OBS * sizeof(double), cudaMemcpyDeviceToHost, st),
+                             "sens gradient read"));
+    uint32_t err = 0;
+    CUDAPIC_CHECK(read_err(s, &err));
+    if (err & CUDAPIC_DEVERR_RECORDS) return fail(CUDAPIC_ERR_CAPACITY, "sens_backward: collision records overflowed");
+    if (err) return fail(CUDAPIC_ERR_CAPACITY, "sens_backward: device error (spawns beyond the capacity)");
     return CUDAPIC_OK;
 }
 

@@ -64,6 +64,34 @@ def test_forward_bit_exact_against_oracle(cudapic, cuda_device, oracle, tables):
     assert obs["ion_flux_gnd"] == pytest.approx(oobs[1], rel=1e-9)
 
 
+@pytest.mark.parametrize("n", [1, 255, 1025, 2_500_000])
+def test_forward_sizes_bit_exact(cudapic, cuda_device, oracle, tables, n):
+    """One ion cycle from a single particle to more rounds per CTA (17 of
+    256 slots) than a 32-bit deposit histogram takes without a drain (15).
+    RNG states bit for bit.  Positions: the FP64 field sums run in another
+    order than the oracle's, so a node's f32 field may round the other way:
+    one ulp of at most 1e6 V/m in each of 20 steps moves a particle by at
+    most 20 dt x 20 x |factor| x 1e6 x 2^-23 = 3e-9 m, and each step rounds
+    x by 2^-24 of the gap (20 x 1.5e-9 m).  A drain that lost or doubled
+    weights would change the charge by its own size."""
+    from cudapic_b200.sensitivity import VoltageSensitivity
+    st, ost, ph = _pair(oracle, n=n)
+    try:
+        with VoltageSensitivity(st, 20, 20) as s:
+            s.forward(V0)
+            info = s.info()
+            got = [s.download(sp) for sp in (0, 1)]
+    finally:
+        st.close()
+    oracle.sens_run(ph, tables, V0, 20, ost, grad=False)
+    assert info["device_error"] == 0 and list(info["slots"]) == list(ost.n)
+    for sp in (0, 1):
+        m = ost.n[sp]
+        np.testing.assert_allclose(got[sp][0][:m], ost.p[sp][0][:m], rtol=0, atol=3.3e-8)
+        for k in range(4):
+            np.testing.assert_array_equal(got[sp][4][k][:m], ost.rng[sp][k][:m])
+
+
 def test_adjoint_against_oracle(cudapic, cuda_device, oracle, tables):
     """d obs / dV0 over 200 steps (checkpoints every 40): f32 tangents with
     FP64 field sums on the GPU against the oracle's double adjoint on the
