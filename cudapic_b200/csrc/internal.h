@@ -89,9 +89,17 @@ struct StepLink {
 // Launchers used by both the drop-in entry points and the driver.
 // zero_a / zero_b (may be null): n_g-float buffers the kernel clears after
 // reading the densities (the driver's next-step density accumulators).
+// meas (cumul_e null: none): the grid quantities of a measured step -- the
+// time-averaged densities (cumul_i on ion steps only) and the XT column of
+// the step (xt may be null) -- added by the solve's own launch; needs a step
+// counter.
+struct PoissonMeasure {
+    double *cumul_e, *cumul_i, *xt;
+    uint32_t n_xt;
+};
 int launch_poisson(const float *e_density, const float *i_density, float *pot, float *efield, float pot0,
                    const float *pot0_table, uint32_t *step_counter, const cudapic_grid &g, cudaStream_t stream,
-                   float *zero_a = nullptr, float *zero_b = nullptr);
+                   float *zero_a = nullptr, float *zero_b = nullptr, const PoissonMeasure &meas = PoissonMeasure{});
 // Adjoint of launch_poisson's solve and field in FP64 (kernels_poisson.cu):
 // eb (field adjoint, cleared) -> neb, nib_acc (density adjoints, the ion one
 // accumulated unless reset_acc) and vbar += cosv * (pot0 adjoint), for `obs`
@@ -160,11 +168,6 @@ enum XtRaw : int {
 int launch_xt_particles(bool ions, const float *x, const float *vx, const float *vy, const float *vz,
                         const uint32_t *n_active, const float *efield, const float *cs, const uint32_t *step_counter,
                         const cudapic_grid &g, uint32_t n_xt, double *xt, cudaStream_t stream);
-// Adds the potential, field and densities of that step.
-int launch_xt_grid(const float *pot, const float *efield, const float *e_density, const float *i_density,
-                   const uint32_t *step_counter, const cudapic_grid &g, uint32_t n_xt, double *xt,
-                   cudaStream_t stream);
-
 // Largest electron / ion collision frequencies of the total tables [1/s]
 // (C/eduPIC.cc:252-276) and the CFL energy limit [eV] (report.cpp).
 void table_coll_freqs(const float *sigma_tot_e, const float *sigma_tot_i, double *max_e, double *max_i);

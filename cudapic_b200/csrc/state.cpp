@@ -247,14 +247,13 @@ int enqueue_step(cudapic_state *s, bool ion_step, bool compact, int next_ion) {
     }
     if (!s->poisson_ahead)  // else the previous step's scatter pass solved it, and cleared the collectors
         CUDAPIC_CHECK(launch_poisson(s->e_density(), s->i_density(), s->pot, s->efield, 0.0f, s->pot0_table,
-                                     s->step_counter(), g, st, e_next, zero_b));
+                                     s->step_counter(), g, st, e_next, zero_b,
+                                     s->measure ? PoissonMeasure{s->cumul_e, ion_step ? s->cumul_i : nullptr, s->xt,
+                                                                 s->n_xt}
+                                                : PoissonMeasure{}));
     s->poisson_ahead = false;
     if (s->measure) {
-        CUDAPIC_CHECK(cudapic_accumulate_density(s->e_density(), s->cumul_e, &g, (cudapic_stream_t)st));
-        if (ion_step) CUDAPIC_CHECK(cudapic_accumulate_density(s->i_density(), s->cumul_i, &g, (cudapic_stream_t)st));
-        if (s->xt) {  // XT diagnostics: the grid of this step and the particles before their push
-            CUDAPIC_CHECK(launch_xt_grid(s->pot, s->efield, s->e_density(), s->i_density(), s->step_counter(), g,
-                                         s->n_xt, s->xt, st));
+        if (s->xt) {  // XT diagnostics: the particles before their push
             CUDAPIC_CHECK(launch_xt_particles(false, s->x[E][se], s->vx[E][se], s->vy[E][se], s->vz[E][se], s->n_e(),
                                               s->efield, s->cs, s->step_counter(), g, s->n_xt, s->xt, st));
             if (ion_step)

@@ -709,3 +709,25 @@ def test_accumulate_eepf_bit_exact(cudapic, K, oracle):
     oracle.accumulate_eepf(x, vx, vy, vz, ef, n, ref, ph)
     assert ref.sum() > 10_000
     assert np.array_equal(host(eepf), ref)
+
+
+@pytest.mark.parametrize("n,shift", [(1, 0), (3, 1), (4, 0), (5, 2), (2047, 3), (2049, 0), (606_209, 0), (606_209, 1)])
+def test_accumulate_eepf_tails_and_alignment(cudapic, K, oracle, n, shift):
+    # four positions per thread, 512 threads, two CTAs per SM: tails of a group, a CTA and the grid, x off 16 bytes
+    import torch
+    from cudapic_b200.workloads import field_profile
+    g = cudapic.grid_from_params(capacity=n + 8)
+    ph = oracle.phys_from_params(capacity=n + 8)
+    x, vx, vy, vz = _population(n, "e", 14, g.dt_e)
+    x = (0.0125 + 0.2 * (x - 0.0125)).astype(np.float32)  # half of them in the central tenth of the gap
+    ef = field_profile(400)
+    eepf = zeros(2000, np.uint32)
+    planes = []
+    for a in (x, vx, vy, vz):
+        t = torch.full((n + 8,), 0.0125, device="cuda")  # past the count: inside the window, not to be sampled
+        t[shift:shift + n] = dev(a)
+        planes.append(t[shift:])
+    K.accumulate_eepf(*planes, dev(ef), counter(n), eepf, g)
+    ref = np.zeros(2000, np.uint32)
+    oracle.accumulate_eepf(x, vx, vy, vz, ef, n, ref, ph)
+    assert np.array_equal(host(eepf), ref)
