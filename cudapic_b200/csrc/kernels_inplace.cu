@@ -60,8 +60,7 @@ __global__ void __launch_bounds__(IP_THREADS, 4)
 // SOLVE: 0, or the last CTA also solves the next step's field (1: FP64
 // scans, 2: f32 scans) with the solve kernel's own shape for N_G <= 1024
 // (one node per thread, so the sums are added in the same order and the
-// field is bit-identical to the separate kernel's): CTAs of 1024 threads,
-// dynamic shared memory n_g x the scan type.
+// field is bit-identical to the separate kernel's): CTAs of 1024 threads.
 constexpr int SC_SOLVE_THREADS = 1024;
 
 template <int SOLVE>
@@ -100,7 +99,7 @@ __global__ void __launch_bounds__(SOLVE ? SC_SOLVE_THREADS : IP_THREADS)
     if (SOLVE) {
         __syncthreads();
         if (s_last)  // every deposit of this step is in: the next step's solve (clears its collectors)
-            poisson_body<typename std::conditional<SOLVE == 1, double, float>::type, 1>(
+            poisson_solve<typename std::conditional<SOLVE == 1, double, float>::type, 1>(
                 ahead.e_density, ahead.i_density, ahead.pot, ahead.efield, 0.0f, ahead.pot0_table,
                 ahead.step_counter, g, ahead.zero_a, ahead.zero_b);
     }
@@ -221,7 +220,7 @@ int launch_electron_scatter(const InplacePlanes &pl, const CollList &list, const
                              stream, pl, list, cs, count, ticket, n_e, n_i, g, dens_e, dens_i, coll, PoissonAhead{});
     if (g.n_g > POISSON_AHEAD_MAX_NG) return fail(CUDAPIC_ERR_ARG, "scatter_colliders_e: n_g too large for the solve");
     const bool f32 = (g.flags & CUDAPIC_FLAG_POISSON_F32_SCAN) != 0;
-    const size_t smem = (size_t)g.n_g * (f32 ? sizeof(float) : sizeof(double));
+    const size_t smem = f32 ? poisson_solve_smem<float>(g.n_g) : poisson_solve_smem<double>(g.n_g);
     const unsigned grid1 = persistent_grid(1, ((uint64_t)g.capacity + SC_SOLVE_THREADS - 1) / SC_SOLVE_THREADS);
     return launch_kernel("scatter_colliders_e+solve_poisson", f32 ? electron_scatter_kernel<2>
                                                                   : electron_scatter_kernel<1>,

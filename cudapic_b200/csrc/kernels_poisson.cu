@@ -2,11 +2,7 @@
 //
 // Reference: solve_poisson_scan_f32, Rust-CUDA/src/main.rs:408-494 (one
 // thread per node, N_G <= 416, f32 block scans) and solve_poisson_dps_flexible,
-// :496-564.  The Dirichlet problem pot[i-1] - 2 pot[i] + pot[i+1] = f_i has
-// unit tridiagonal coefficients, so the Thomas recurrences collapse to
-//     G_i = sum_{j<=i} j f_j,   r_i = -G_i / ((i+1) i),   pot_i = i sum_{j=i}^{N-2} r_j,
-// i.e. two inclusive prefix sums (C/eduPIC.cc:461-494 is the sequential
-// Thomas form of the same system).
+// :496-564.  The closed forms are derived in poisson.cuh.
 //
 // B200 design: one CTA of up to 1024 threads, each thread owning
 // ceil(N_G / blockDim) consecutive nodes (N_G up to 16384), warp-shuffle
@@ -93,7 +89,7 @@ __global__ void __launch_bounds__(POIS_MAX_THREADS)
     grid_dep_wait();
     MeasureGrid mg;
     mg.fetch(meas, step_counter, g);
-    poisson_body<T, PT>(e_density, i_density, pot_out, efield_out, pot0_arg, pot0_table, step_counter, g, zero_a,
+    poisson_solve<T, PT>(e_density, i_density, pot_out, efield_out, pot0_arg, pot0_table, step_counter, g, zero_a,
                         zero_b);
     mg.add(meas, e_density, i_density, pot_out, efield_out, g);
 }
@@ -174,7 +170,7 @@ template <typename T, int PT>
 int launch_poisson_t(const float *e_density, const float *i_density, float *pot, float *efield, float pot0,
                      const float *pot0_table, uint32_t *step_counter, const cudapic_grid &g, int threads,
                      cudaStream_t stream, float *zero_a, float *zero_b, const PoissonMeasure &meas) {
-    size_t smem = (size_t)g.n_g * sizeof(T);
+    const size_t smem = poisson_solve_smem<T>(g.n_g);
     auto kern = poisson_kernel<T, PT>;
     if (smem > 48 * 1024)
         CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
@@ -465,7 +461,7 @@ __global__ void __launch_bounds__(POIS_MAX_THREADS)
                                         : PoissonMeasure{};
     MeasureGrid mg;
     mg.fetch(meas, ctr + 3, s_g);
-    poisson_body<T, PT>(e_dens, i_dens, dd.pot, dd.efield, 0.0f, dd.pot0_table, ctr + 3, s_g, dd.e_dens[e_read ^ 1],
+    poisson_solve<T, PT>(e_dens, i_dens, dd.pot, dd.efield, 0.0f, dd.pot0_table, ctr + 3, s_g, dd.e_dens[e_read ^ 1],
                         ion_step ? dd.i_dens[i_read ^ 1] : nullptr);
     mg.add(meas, e_dens, i_dens, dd.pot, dd.efield, s_g);
 }
@@ -473,7 +469,7 @@ __global__ void __launch_bounds__(POIS_MAX_THREADS)
 template <typename T, int PT>
 int launch_batch_poisson_t(const BatchDisc *desc, uint32_t *counts, uint32_t D, uint32_t max_n_g, int threads,
                            int e_read, int i_read, int ion_step, int measure, cudaStream_t stream) {
-    const size_t smem = (size_t)max_n_g * sizeof(T);
+    const size_t smem = poisson_solve_smem<T>(max_n_g);
     auto kern = batch_poisson_kernel<T, PT>;
     if (smem > 48 * 1024)
         CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),

@@ -696,6 +696,26 @@ def test_spawn_capacity_is_enforced(cudapic, K, oracle, dev_tables, tables):
 
 # ---------------------------------------------------------------- diagnostics
 
+@pytest.mark.parametrize("n_g", [3, 4, 5, 31, 32, 33, 1023, 1024, 1026, 2048, 2051, 4097, 8191, 12289, 16383])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_poisson_fp64_edges(cudapic, K, oracle, n_g, shift):
+    """Ends of a warp, of the nodes per thread (1 .. 16) and of the largest
+    grid, densities on and off 16 bytes, against the FP64 Thomas solve.  The
+    outputs are rounded to f32 (2^-24 relative each); the FP64 sums add at
+    most n_g 2^-53 of sums that exceed the result by up to n_g: below 2^-24
+    for n_g <= 16384.  2^-22 leaves a factor four."""
+    g = cudapic.grid_from_params(n_g=n_g)
+    ph = oracle.phys_from_params(n_g=n_g)
+    ne, ni = _profile(n_g, n_g)
+    pot, ef = zeros(n_g), zeros(n_g)
+    pad = np.zeros(shift, np.float32)
+    e, i = dev(np.concatenate([pad, ne])), dev(np.concatenate([pad, ni]))
+    K.solve_poisson_scan_f32(e[shift:], i[shift:], pot, ef, 250.0, g)
+    rp, re = oracle.poisson_thomas_f64(ne, ni, 250.0, ph)
+    assert np.linalg.norm(host(pot) - rp) <= 2.0 ** -22 * np.linalg.norm(rp)
+    assert np.linalg.norm(host(ef) - re) <= 2.0 ** -22 * np.linalg.norm(re)
+
+
 def test_accumulate_eepf_bit_exact(cudapic, K, oracle):
     from cudapic_b200.workloads import field_profile
     n = 500_000
