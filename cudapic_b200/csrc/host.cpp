@@ -5,9 +5,11 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <thread>
+#include <tuple>
 #include <vector>
 
 #include "internal.h"
@@ -63,6 +65,94 @@ int check_launch(const char *kernel) {
 
 int sm_count() { return device_info().sms; }
 int max_smem_optin() { return device_info().smem_optin; }
+
+namespace {
+// Identity of the calling thread's context (never reused, so that a context
+// created after a cudaDeviceReset, or one of the caller's own, gets its own
+// entries); 0 when there is none yet or the driver cannot tell: nothing is
+// kept then.
+unsigned long long context_id() {
+    using Fn = int (*)(void *, unsigned long long *);
+    static const Fn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return reinterpret_cast<Fn>(p);
+    }();
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == 0 ? id + 1 : 0;
+}
+
+using LimitKey = std::tuple<unsigned long long, const void *, int, size_t, int>;  // context, kernel, threads, smem, cluster
+std::mutex g_limit_mu;
+std::map<LimitKey, int> g_limits;
+std::map<std::pair<unsigned long long, const void *>, size_t> g_smem_limit;
+constexpr size_t MAX_LIMITS = 4096;  // shapes kept (a sweep over grids meets a few per kernel)
+// Every launch may take 48 KB of static and dynamic shared memory together;
+// the kernels' static part is below 16 KB.
+constexpr size_t FREE_SMEM = 32 * 1024;
+
+// The kept answer for a shape, or that of `query` (which may fail).
+template <typename Query>
+int kept_limit(const void *kern, int threads, size_t smem, int cluster, int *out, Query query) {
+    const unsigned long long ctx = context_id();
+    const LimitKey key{ctx, kern, threads, smem, cluster};
+    std::lock_guard<std::mutex> lk(g_limit_mu);
+    if (ctx) {
+        const auto it = g_limits.find(key);
+        if (it != g_limits.end()) {
+            *out = it->second;
+            return CUDAPIC_OK;
+        }
+    }
+    size_t &limit = g_smem_limit[{ctx, kern}];
+    if (smem > FREE_SMEM && (!ctx || smem > limit)) {
+        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                                 "cudaFuncSetAttribute"));
+        limit = smem;
+    }
+    CUDAPIC_CHECK(query());
+    if (ctx) {
+        if (g_limits.size() >= MAX_LIMITS) g_limits.clear();
+        g_limits[key] = *out;
+    }
+    return CUDAPIC_OK;
+}
+}  // namespace
+
+int kernel_smem(const void *kern, size_t smem, const char *what) {
+    if (smem <= FREE_SMEM) return CUDAPIC_OK;
+    int unused = 0;
+    const int rc = kept_limit(kern, 0, smem, 0, &unused, [] { return CUDAPIC_OK; });
+    return rc == CUDAPIC_OK ? rc : fail(rc, std::string(what) + ": " + g_last_error);
+}
+
+int kernel_blocks(const void *kern, int threads, size_t smem, int *per_sm, const char *what) {
+    return kept_limit(kern, threads, smem, 0, per_sm, [&] {
+        return check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, threads, smem), what);
+    });
+}
+
+int kernel_clusters(const void *kern, int threads, size_t smem, int cluster, int *clusters, const char *what) {
+    return kept_limit(kern, threads, smem, cluster, clusters, [&] {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)cluster;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(cluster * 64);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return check_cuda(cudaOccupancyMaxActiveClusters(clusters, kern, &cfg), what);
+    });
+}
 
 namespace {
 // Built-in launch shapes (chosen with cudapic_b200.autotune on B200).

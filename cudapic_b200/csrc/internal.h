@@ -27,6 +27,18 @@ int max_smem_optin();
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Launch limits of a kernel in the current context, asked of the runtime once
+// per shape and context and kept (the queries cost a drop-in call more than
+// its launch: cudaFuncSetAttribute with cudaOccupancyMaxActiveBlocks 2 us,
+// cudaOccupancyMaxActiveClusters 4 us).
+//  kernel_smem: lets launches of `kern` take `smem` bytes of dynamic shared
+//    memory (the limit is only ever raised);
+//  kernel_blocks: the same, and the resident CTAs per SM of that shape;
+//  kernel_clusters: the same, and the resident clusters of `cluster` CTAs.
+int kernel_smem(const void *kern, size_t smem, const char *what);
+int kernel_blocks(const void *kern, int threads, size_t smem, int *per_sm, const char *what);
+int kernel_clusters(const void *kern, int threads, size_t smem, int cluster, int *clusters, const char *what);
+
 // Validation shared by the entry points.
 int validate_grid(const cudapic_grid *g);
 

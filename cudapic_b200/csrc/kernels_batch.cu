@@ -557,10 +557,7 @@ int launch_batch_step_t(const StepPlanes &pl, const BatchDisc *desc, const uint3
     auto kern = batch_step_kernel<U, MCC, MINB, MEAS>;
     int per_sm = 0;
     auto occupancy = [&]() {
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes()),
-                                 "cudaFuncSetAttribute(batch step)"));
-        return check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ES_THREADS, bytes()),
-                          "occupancy(batch step)");
+        return kernel_blocks((const void *)kern, ES_THREADS, bytes(), &per_sm, "occupancy(batch step)");
     };
     CUDAPIC_CHECK(occupancy());
     // large grids: fewer histogram copies rather than fewer CTAs per SM
@@ -621,10 +618,7 @@ int launch_batch_inplace(const InplacePlanes &pl, const CollList &list, const Ba
     auto kern = r.measure ? batch_inplace_kernel<true> : batch_inplace_kernel<false>;
     int per_sm = 0;
     auto occupancy = [&]() {
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes()),
-                                 "cudaFuncSetAttribute(batch in-place step)"));
-        return check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, IP_THREADS, bytes()),
-                          "occupancy(batch in-place step)");
+        return kernel_blocks((const void *)kern, IP_THREADS, bytes(), &per_sm, "occupancy(batch in-place step)");
     };
     CUDAPIC_CHECK(occupancy());
     // large grids: fewer copies rather than fewer CTAs; below 4 copies the

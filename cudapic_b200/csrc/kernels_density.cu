@@ -242,8 +242,6 @@ namespace {
 template <typename Kern, typename... Args>
 int launch_clustered(Kern kern, int block, size_t smem, const cudapic_grid &g, const cudapic_tuning &t,
                      cudaStream_t stream, Args... args) {
-    CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                             "cudaFuncSetAttribute(get_density)"));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -257,9 +255,8 @@ int launch_clustered(Kern kern, int block, size_t smem, const cudapic_grid &g, c
     cfg.numAttrs = 1;
     const int cl = t.density_cluster;
     int max_clusters = 0;
-    cfg.gridDim = dim3(cl * 64);
-    CUDAPIC_CHECK(check_cuda(cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg),
-                             "cudaOccupancyMaxActiveClusters(get_density)"));
+    CUDAPIC_CHECK(kernel_clusters((const void *)kern, block, smem, cl, &max_clusters,
+                                  "cudaOccupancyMaxActiveClusters(get_density)"));
     if (max_clusters < 1) return fail(CUDAPIC_ERR_NOT_SUPPORTED, "get_density: no resident cluster");
     const uint64_t want = (uint64_t)sm_count() * (uint64_t)t.density_ctas_per_sm / (uint64_t)cl;
     const uint64_t need = ((uint64_t)g.capacity + 4ull * block - 1) / (4ull * block);

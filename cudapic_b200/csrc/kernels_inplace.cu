@@ -183,11 +183,8 @@ int launch_electron_inplace(const InplacePlanes &pl, const float *efield, const 
     auto kern = wall ? electron_inplace_kernel<true> : electron_inplace_kernel<false>;
     int per_sm = 0;
     auto occupancy = [&]() {
-        const size_t smem = inplace_smem_bytes(copies, ef_pad);
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                                 "cudaFuncSetAttribute(step_electrons_inplace)"));
-        return check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, IP_THREADS, smem),
-                          "occupancy(step_electrons_inplace)");
+        return kernel_blocks((const void *)kern, IP_THREADS, inplace_smem_bytes(copies, ef_pad), &per_sm,
+                             "occupancy(step_electrons_inplace)");
     };
     CUDAPIC_CHECK(occupancy());
     // large grids: fewer copies rather than fewer CTAs; below 4 copies the

@@ -414,11 +414,8 @@ int launch_tma(const float *sigma_tot, const float *cs, const uint32_t *active, 
     const cudapic_tuning t = tuning();
     const int stages = std::min(std::max(t.mcc_stages, 2), MT_MAX_STAGES);
     const size_t smem = mcc_tma_smem_bytes(stages);
-    CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                             "cudaFuncSetAttribute(check_collisions)"));
     int per_sm = 0;
-    CUDAPIC_CHECK(check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MCC_THREADS, smem),
-                             "occupancy(check_collisions)"));
+    CUDAPIC_CHECK(kernel_blocks((const void *)kern, MCC_THREADS, smem, &per_sm, "occupancy(check_collisions)"));
     per_sm = std::min(std::max(per_sm, 1), t.mcc_ctas_per_sm);
     const uint64_t tiles_max = ((uint64_t)g.capacity + MT_TILE - 1) / MT_TILE;
     const unsigned grid = persistent_grid(per_sm, tiles_max);
@@ -435,8 +432,7 @@ int launch_resident(const float *sigma_tot, const float *cs, const uint32_t *act
                     unsigned long long *coll, float ion_k) {
     auto kern = check_collisions_resident_kernel<ION, EVENTS>;
     if (MR_SMEM > (size_t)max_smem_optin()) return fail(CUDAPIC_ERR_NOT_SUPPORTED, "check_collisions: shared memory");
-    CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MR_SMEM),
-                             "cudaFuncSetAttribute(check_collisions resident)"));
+    CUDAPIC_CHECK(kernel_smem((const void *)kern, MR_SMEM, "check_collisions"));
     const uint64_t chunks = ((uint64_t)g.capacity + MR_THREADS * MR_U - 1) / (MR_THREADS * MR_U);
     return launch_kernel(ION ? "check_collisions_i" : "check_collisions_e", kern, dim3(persistent_grid(1, chunks)),
                          dim3(MR_THREADS), MR_SMEM, stream, sigma_tot, cs, active, x, vx, vy, vz, r0, r1, r2, r3, ix,

@@ -236,9 +236,7 @@ extern "C" int cudapic_xoshiro128_seed_streams(const uint32_t master[4], uint32_
     const uint32_t per_thread = (n + step - 1) / step;
     const uint32_t block = SEED_THREADS * per_thread;
     const size_t smem = per_thread > 1 ? SEED_TABLE_BYTES : 0;
-    if (smem)
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(seed_streams_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                      (int)smem), "cudaFuncSetAttribute(xoshiro128_seed_streams)"));
+    CUDAPIC_CHECK(kernel_smem((const void *)seed_streams_kernel, smem, "xoshiro128_seed_streams"));
     seed_streams_kernel<<<(n + block - 1) / block, SEED_THREADS, smem, (cudaStream_t)stream>>>(m, n, per_thread, rng0,
                                                                                               rng1, rng2, rng3);
     return check_launch("xoshiro128_seed_streams");

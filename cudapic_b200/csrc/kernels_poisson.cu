@@ -172,9 +172,7 @@ int launch_poisson_t(const float *e_density, const float *i_density, float *pot,
                      cudaStream_t stream, float *zero_a, float *zero_b, const PoissonMeasure &meas) {
     const size_t smem = poisson_solve_smem<T>(g.n_g);
     auto kern = poisson_kernel<T, PT>;
-    if (smem > 48 * 1024)
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                                 "cudaFuncSetAttribute(poisson)"));
+    CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "poisson"));
     return launch_kernel("solve_poisson_scan", kern, dim3(1), dim3(threads), smem, stream, e_density, i_density, pot,
                          efield, pot0, pot0_table, step_counter, g, zero_a, zero_b, meas);
 }
@@ -292,9 +290,7 @@ int launch_poisson_adjoint_t(double *eb, double *neb, double *nib_acc, int reset
                              int obs, const cudapic_grid &g, int threads, cudaStream_t stream) {
     const size_t smem = (size_t)g.n_g * sizeof(double);
     auto kern = poisson_adjoint_kernel<PT>;
-    if (smem > 48 * 1024)
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                                 "cudaFuncSetAttribute(poisson_adjoint)"));
+    CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "poisson_adjoint"));
     return launch_kernel("poisson_adjoint", kern, dim3(obs), dim3(threads), smem, stream, eb, neb, nib_acc, reset_acc,
                          cosv, vbar, g);
 }
@@ -404,9 +400,7 @@ int launch_poisson_f64_t(const double *dens_e, const double *dens_i, double *pot
                          double *pot_sum, const cudapic_grid &g, int threads, cudaStream_t stream) {
     const size_t smem = (size_t)g.n_g * sizeof(double);
     auto kern = poisson_f64_kernel<PT>;
-    if (smem > 48 * 1024)
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                                 "cudaFuncSetAttribute(poisson_f64)"));
+    CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "poisson_f64"));
     return launch_kernel("poisson_f64", kern, dim3(1), dim3(threads), smem, stream, dens_e, dens_i, pot, efield,
                          pot0_table, step, ion_step, cumul_e, cumul_i, pot_sum, g);
 }
@@ -471,9 +465,7 @@ int launch_batch_poisson_t(const BatchDisc *desc, uint32_t *counts, uint32_t D, 
                            int e_read, int i_read, int ion_step, int measure, cudaStream_t stream) {
     const size_t smem = poisson_solve_smem<T>(max_n_g);
     auto kern = batch_poisson_kernel<T, PT>;
-    if (smem > 48 * 1024)
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                                 "cudaFuncSetAttribute(batch poisson)"));
+    CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "batch poisson"));
     return launch_kernel("batch_solve_poisson", kern, dim3(D), dim3(threads), smem, stream, desc, counts, D, e_read,
                          i_read, ion_step, measure);
 }

@@ -329,10 +329,7 @@ int launch_move_and_compact(const float *efield, const float *sx, const float *s
         auto kern = dep ? move_and_compact_tma_kernel<true> : move_and_compact_tma_kernel<false>;
         int per_sm = 0;
         auto occupancy = [&]() {
-            CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                                     "cudaFuncSetAttribute(move_and_compact)"));
-            return check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MC_THREADS, smem),
-                              "occupancy(move_and_compact)");
+            return kernel_blocks((const void *)kern, MC_THREADS, smem, &per_sm, "occupancy(move_and_compact)");
         };
         CUDAPIC_CHECK(occupancy());
         // large grids: fewer histogram copies rather than fewer CTAs per SM
@@ -364,10 +361,7 @@ int launch_move_and_compact(const float *efield, const float *sx, const float *s
         return CUDAPIC_OK;
     }
     const size_t smem = (size_t)g.n_g * sizeof(float);
-    if (smem > 48 * 1024)
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(move_and_compact_simple_kernel,
-                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                                 "cudaFuncSetAttribute(move_and_compact_simple)"));
+    CUDAPIC_CHECK(kernel_smem((const void *)move_and_compact_simple_kernel, smem, "move_and_compact_simple"));
     const uint64_t blocks_max = ((uint64_t)g.capacity + MCS_THREADS - 1) / MCS_THREADS;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sm_count() * 4, blocks_max));
     return launch_kernel("move_and_compact_simple", move_and_compact_simple_kernel, dim3(grid), dim3(MCS_THREADS), smem,

@@ -144,10 +144,7 @@ int launch_electron_step_t(const float *efield, const float *sx, const float *sv
     auto kern = electron_step_kernel<U>;
     int per_sm = 0;
     auto occupancy = [&]() {
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes()),
-                                 "cudaFuncSetAttribute(step_electrons)"));
-        return check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ES_THREADS, bytes()),
-                          "occupancy(step_electrons)");
+        return kernel_blocks((const void *)kern, ES_THREADS, bytes(), &per_sm, "occupancy(step_electrons)");
     };
     CUDAPIC_CHECK(occupancy());
     // large grids: fewer histogram copies rather than fewer CTAs per SM (the

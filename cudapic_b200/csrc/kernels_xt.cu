@@ -193,8 +193,7 @@ int launch_xt_particles(bool ions, const float *x, const float *vx, const float 
     const size_t smem = (size_t)(ions ? 3 : 4) * g.n_g * sizeof(float);
     if (smem > (size_t)max_smem_optin()) return fail(CUDAPIC_ERR_ARG, "xt: n_g too large");
     auto kern = ions ? xt_particles_kernel<true> : xt_particles_kernel<false>;
-    CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                             "cudaFuncSetAttribute(xt)"));
+    CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "xt"));
     const unsigned grid = persistent_grid(1, ((uint64_t)g.capacity + XT_THREADS - 1) / XT_THREADS);
     return launch_kernel(ions ? "xt_ions" : "xt_electrons", kern, dim3(grid), dim3(XT_THREADS), smem, stream, x, vx,
                          vy, vz, n_active, efield, cs, step_counter, g, n_xt, xt);
@@ -207,8 +206,7 @@ int launch_batch_xt_particles(bool ions, const SidePlanes &sp, const BatchDisc *
     if (smem > (size_t)max_smem_optin() - sizeof(uint32_t) * (BATCH_MAX_DISCHARGES + 1))
         return fail(CUDAPIC_ERR_ARG, "batch xt: n_g too large");
     auto kern = ions ? batch_xt_particles_kernel<true> : batch_xt_particles_kernel<false>;
-    CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                             "cudaFuncSetAttribute(batch xt)"));
+    CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "batch xt"));
     const unsigned grid = persistent_grid(1, (cap_sum + XT_THREADS - 1) / XT_THREADS);
     return launch_kernel(ions ? "batch_xt_ions" : "batch_xt_electrons", kern, dim3(grid), dim3(XT_THREADS), smem,
                          stream, sp, desc, D);

@@ -28,13 +28,25 @@ def _ptr(t):
     return t.data_ptr()
 
 
-def _stream(stream, *tensors):
+_current_stream = None
+
+
+def _stream_getter():
+    """torch's current stream of a device index as an address: the raw getter
+    where torch has one (building a Stream object costs as much as a launch)."""
+    import torch
+    return (getattr(torch._C, "_cuda_getCurrentRawStream", None)
+            or (lambda index: torch.cuda.current_stream(index).cuda_stream))
+
+
+def _stream(stream, t):
     if stream is not None:
         return stream if isinstance(stream, int) else stream.cuda_stream
-    for t in tensors:
-        if hasattr(t, "is_cuda") and t.is_cuda:
-            import torch
-            return torch.cuda.current_stream(t.device).cuda_stream
+    if getattr(t, "is_cuda", False):
+        global _current_stream
+        if _current_stream is None:
+            _current_stream = _stream_getter()
+        return _current_stream(t.get_device())
     return 0
 
 
