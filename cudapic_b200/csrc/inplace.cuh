@@ -356,8 +356,8 @@ __device__ __forceinline__ void inplace_scatter(const InplacePlanes &pl, const C
     const float xi = (w >> 31) ? pl.x[j] : 0.0f;  // an ionization's birthplace, fetched beside the table lookups
     const float v2 = vxi * vxi + vyi * vyi + vzi * vzi;
     const uint32_t idx = energy_index(g.half_me_over_e * v2);
-    collide_electron_body<true, true>(off, i, idx, vxi, vyi, vzi, rs, cs, pl.x, pl.vx, pl.vy, pl.vz, pl.ix, pl.ivx,
-                                      pl.ivy, pl.ivz, n_e, n_i, g, dens_e, dens_i, xi);
+    const SpawnToPlanes spawn{off, pl.x, pl.vx, pl.vy, pl.vz, pl.ix, pl.ivx, pl.ivy, pl.ivz, n_e, n_i, dens_e, dens_i, g};
+    collide_electron_body<true, true>(j, idx, vxi, vyi, vzi, rs, cs, pl.x, pl.vx, pl.vy, pl.vz, g, spawn, xi);
 }
 
 }  // namespace cudapic

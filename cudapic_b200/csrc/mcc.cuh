@@ -165,27 +165,57 @@ __device__ __forceinline__ void deposit_global(float *dens, float xv, const cuda
     atomicAdd(&dens[p + 1], c2);
 }
 
-// collision_e, Rust-CUDA/src/main.rs:1035-1165: scatters electron i (state
-// rs already past the test draw), writes its velocity and any spawns;
-// returns the event (1 elastic, 2 excitation, 3 ionization).  dep_e / dep_i
-// (may be null): next-step densities that also receive the spawned
-// electron / ion.  Slots (i and the spawns' claimed slots) are relative to
-// element `off` of the planes (a discharge of a batch's pool; 0 otherwise).
+// The spawns of an ionization in global planes: each claims the next slot of
+// its species' counter (relative to element `off`; dropped and flagged beyond
+// the capacity) and is deposited into the next-step density (may be null).
+struct SpawnToPlanes {
+    uint32_t off;
+    float *x, *vx, *vy, *vz, *ix, *ivx, *ivy, *ivz;
+    uint32_t *alive_e, *alive_i;
+    float *dep_e, *dep_i;
+    const cudapic_grid &g;
+    __device__ __forceinline__ void electron(float xi, float a, float b, float c) const {
+        uint32_t slot;
+        if (claim_slot(alive_e, g.capacity, slot)) {
+            x[off + slot] = xi;
+            vx[off + slot] = a;
+            vy[off + slot] = b;
+            vz[off + slot] = c;
+            if (dep_e) deposit_global(dep_e, xi, g);
+        } else {
+            set_dev_err(g.dev_err, CUDAPIC_DEVERR_SPAWN_E);
+        }
+    }
+    __device__ __forceinline__ void ion(float xi, float a, float b, float c) const {
+        uint32_t slot;
+        if (claim_slot(alive_i, g.capacity, slot)) {
+            ix[off + slot] = xi;
+            ivx[off + slot] = a;
+            ivy[off + slot] = b;
+            ivz[off + slot] = c;
+            if (dep_i) deposit_global(dep_i, xi, g);
+        } else {
+            set_dev_err(g.dev_err, CUDAPIC_DEVERR_SPAWN_I);
+        }
+    }
+};
+
+// collision_e, Rust-CUDA/src/main.rs:1035-1165: scatters an electron (state
+// rs already past the test draw), writes its velocity to vx[j], vy[j], vz[j]
+// and hands any spawns to `spawn` (SpawnToPlanes); returns the event (1
+// elastic, 2 excitation, 3 ionization).
 // ALG: the sines and cosines of the Euler angles, of the scattering angles
 // chi = acos(c) and of eta + pi from their algebraic forms (euler_angles_alg,
 // sincos_of_acos, sin(eta + pi) = -sin eta) instead of evaluating the
 // angles: the same draws and events, velocities equal up to the rounding of
 // the skipped transcendentals, a fraction of the arithmetic.
 // XPRE: the caller passes the electron's position as xpre (loaded ahead,
-// alongside its other loads); else an ionization loads x[off + i] itself.
-template <bool ALG, bool XPRE>
-__device__ __forceinline__ uint32_t collide_electron_body(uint32_t off, uint32_t i, uint32_t idx, float vxi,
-                                                          float vyi, float vzi, Xoshiro128p &rs,
-                                                          const float *__restrict__ cs, float *x, float *vx,
-                                                          float *vy, float *vz, float *ix, float *ivx, float *ivy,
-                                                          float *ivz, uint32_t *alive_e, uint32_t *alive_i,
-                                                          const cudapic_grid &g, float *dep_e, float *dep_i,
-                                                          float xpre) {
+// alongside its other loads); else an ionization loads x[j] itself.
+template <bool ALG, bool XPRE, typename Spawn>
+__device__ __forceinline__ uint32_t collide_electron_body(uint32_t j, uint32_t idx, float vxi, float vyi, float vzi,
+                                                          Xoshiro128p &rs, const float *__restrict__ cs,
+                                                          const float *x, float *vx, float *vy, float *vz,
+                                                          const cudapic_grid &g, const Spawn &spawn, float xpre) {
     const float exc_j = 11.5f * E_CHARGE_F;
     const float ion_j = 15.8f * E_CHARGE_F;
     float gx = vxi, gy = vyi, gz = vzi;
@@ -235,42 +265,27 @@ __device__ __forceinline__ uint32_t collide_electron_body(uint32_t off, uint32_t
         }
         float ngx, ngy, ngz;
         rotate(g_new, sc2, cc2, se2, ce2, eu, ngx, ngy, ngz);
-        const float xi = XPRE ? xpre : x[off + i];
-        uint32_t slot;
-        if (claim_slot(alive_e, g.capacity, slot)) {
-            x[off + slot] = xi;
-            vx[off + slot] = wx + g.f2 * ngx;
-            vy[off + slot] = wy + g.f2 * ngy;
-            vz[off + slot] = wz + g.f2 * ngz;
-            if (dep_e) deposit_global(dep_e, xi, g);
-        } else {
-            set_dev_err(g.dev_err, CUDAPIC_DEVERR_SPAWN_E);
-        }
+        const float xi = XPRE ? xpre : x[j];
+        spawn.electron(xi, wx + g.f2 * ngx, wy + g.f2 * ngy, wz + g.f2 * ngz);
         float a, b, c;
         rs.three_normal(g.normal_range, a, b, c);
-        if (claim_slot(alive_i, g.capacity, slot)) {
-            ix[off + slot] = xi;
-            ivx[off + slot] = a;
-            ivy[off + slot] = b;
-            ivz[off + slot] = c;
-            if (dep_i) deposit_global(dep_i, xi, g);
-        } else {
-            set_dev_err(g.dev_err, CUDAPIC_DEVERR_SPAWN_I);
-        }
+        spawn.ion(xi, a, b, c);
         if (ALG) sincos_of_acos(sqrtf(e_orig / en), &chi_s, &chi_c);
         else dm::sincosf_det(dm::acosf_det(sqrtf(e_orig / en)), &chi_s, &chi_c);
     }
     if (!ALG || ev != 3) dm::sincosf_det(eta, &se, &ce);
     float ngx, ngy, ngz;
     rotate(gm, chi_s, chi_c, se, ce, eu, ngx, ngy, ngz);
-    vx[off + i] = wx + g.f2 * ngx;
-    vy[off + i] = wy + g.f2 * ngy;
-    vz[off + i] = wz + g.f2 * ngz;
+    vx[j] = wx + g.f2 * ngx;
+    vy[j] = wy + g.f2 * ngy;
+    vz[j] = wz + g.f2 * ngz;
     return ev;
 }
 
-// The body as one out-of-line function: the callers that run it inside a
-// streaming loop keep its registers out of their own.
+// The body over global planes as one out-of-line function (electron i and the
+// spawns' slots relative to element `off`, a discharge of a batch's pool; 0
+// otherwise): the callers that run it inside a streaming loop keep its
+// registers out of their own.
 template <bool ALG>
 static __device__ __noinline__ uint32_t collide_electron_t(uint32_t off, uint32_t i, uint32_t idx, float vxi,
                                                     float vyi, float vzi, Xoshiro128p &rs,
@@ -278,8 +293,8 @@ static __device__ __noinline__ uint32_t collide_electron_t(uint32_t off, uint32_
                                                     float *vz, float *ix, float *ivx, float *ivy, float *ivz,
                                                     uint32_t *alive_e, uint32_t *alive_i, const cudapic_grid &g,
                                                     float *dep_e, float *dep_i) {
-    return collide_electron_body<ALG, false>(off, i, idx, vxi, vyi, vzi, rs, cs, x, vx, vy, vz, ix, ivx, ivy, ivz,
-                                             alive_e, alive_i, g, dep_e, dep_i, 0.0f);
+    const SpawnToPlanes spawn{off, x, vx, vy, vz, ix, ivx, ivy, ivz, alive_e, alive_i, dep_e, dep_i, g};
+    return collide_electron_body<ALG, false>(off + i, idx, vxi, vyi, vzi, rs, cs, x, vx, vy, vz, g, spawn, 0.0f);
 }
 
 // The reference formulation (the drop-in collision kernels).

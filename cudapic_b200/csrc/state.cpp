@@ -27,6 +27,7 @@
 
 #include "batch_internal.h"
 #include "internal.h"
+#include "resident.h"
 #include "state_impl.h"
 
 namespace {
@@ -352,6 +353,64 @@ int build_graph(cudapic_state *s) {
     cudaGraphDestroy(graph);
     s->graph_gen[m] = tuning_generation();
     return check_cuda(e, "cudaGraphInstantiate");
+}
+
+// Steps of one resident launch at most (a few milliseconds).
+constexpr uint64_t RESIDENT_MAX_STEPS = 1000;
+
+// Whether the next steps run in the resident kernel: the driver's default
+// steps of a discharge that fits it, whole ion cycles.
+bool use_resident(const cudapic_state *s, uint64_t n_steps) {
+    const uint64_t n_sub = s->params.n_sub;
+    if (!s->fused || !s->inplace || !s->overlap || !s->solve_ahead || !s->graphs_enabled || s->spawn_collide ||
+        s->measure || s->steps_done % n_sub != 0 || n_steps < n_sub || !resident_fits(s->grid, s->params.n_sub))
+        return false;
+    const void *planes[8] = {s->x[1][0], s->vx[1][0], s->vy[1][0], s->vz[1][0],
+                             s->x[1][1], s->vx[1][1], s->vy[1][1], s->vz[1][1]};
+    return electron_step_eligible(planes, 8, s->grid.capacity);
+}
+
+// Enqueues `steps` steps (whole ion cycles) as one launch and moves the
+// buffer roles on: each ion cycle flips the ions' side and densities, each
+// step the electron densities (the electrons return to their side).
+int enqueue_resident(cudapic_state *s, uint32_t steps) {
+    if (!s->dens_valid) CUDAPIC_CHECK(state_prime_fused(s, s->stream));
+    const int odd_cycles = (int)(steps / s->params.n_sub & 1u);
+    const int e_cur = s->e_cur ^ (int)(steps & 1u), i_cur = s->i_cur ^ odd_cycles;
+    ResidentArgs a{};
+    const int se = s->side[0];
+    a.e = {s->x[0][se], s->vx[0][se], s->vy[0][se], s->vz[0][se]};
+    for (int k = 0; k < 2; ++k) {
+        const int si = s->side[1] ^ k;
+        a.i[k] = {s->x[1][si], s->vx[1][si], s->vy[1][si], s->vz[1][si]};
+    }
+    for (int k = 0; k < 4; ++k) {
+        a.rng_e[k] = s->rng[0][k];
+        a.rng_i[k] = s->rng[1][k];
+    }
+    a.n_e = s->n_e();
+    a.n_i = s->n_i();
+    a.alive_i = s->alive_i();
+    a.step_counter = s->step_counter();
+    a.n_sub = s->params.n_sub;
+    a.e_dens_in = s->e_dens[s->e_cur];
+    a.i_collected = s->i_dens[s->i_cur ^ 1];
+    a.e_dens_out = s->e_dens[e_cur];
+    a.i_current_out = s->i_dens[i_cur];
+    a.i_collected_out = s->i_dens[i_cur ^ 1];
+    a.pot = s->pot;
+    a.efield = s->efield;
+    a.pot0_table = s->pot0_table;
+    a.sigma_tot_e = s->sigma_tot_e;
+    a.sigma_tot_i = s->sigma_tot_i;
+    a.cs = s->cs;
+    a.sigma_max = s->sigma_max_e;
+    a.ion_k = s->ion_k;
+    CUDAPIC_CHECK(launch_resident(a, s->grid, steps, s->stream));
+    s->side[1] ^= odd_cycles;
+    s->e_cur = e_cur;
+    s->i_cur = i_cur;
+    return CUDAPIC_OK;
 }
 
 }  // namespace
@@ -736,6 +795,14 @@ extern "C" int cudapic_state_run_steps(cudapic_state *s, uint64_t n_steps) {
     DeviceGuard dg(s->device);
     const uint64_t period = graph_period(s);
     while (n_steps > 0) {
+        if (use_resident(s, n_steps)) {
+            const uint64_t n_sub = s->params.n_sub;
+            const uint64_t steps = std::max(n_sub, std::min(n_steps, RESIDENT_MAX_STEPS) / n_sub * n_sub);
+            CUDAPIC_CHECK(enqueue_resident(s, (uint32_t)steps));
+            s->steps_done += steps;
+            n_steps -= steps;
+            continue;
+        }
         const bool primed = !s->fused || s->dens_valid;  // a priming step is never captured
         if (s->graphs_enabled && primed && (s->steps_done % period) == 0 && n_steps >= period) {
             const int m = s->measure ? 1 : 0;
