@@ -63,8 +63,12 @@ __global__ void __launch_bounds__(IP_THREADS, 4)
 // field is bit-identical to the separate kernel's): CTAs of 1024 threads.
 constexpr int SC_SOLVE_THREADS = 1024;
 
+// 40 registers: 1024 threads then leave 24 K of an SM's registers, and under
+// programmatic dependent launch a CTA of the next step's stream pass (16 K)
+// is already there when the solve ends (at 49 registers 400 steps of 4.2 M
+// electrons took 26.2 ms, at 40 25.9).
 template <int SOLVE>
-__global__ void __launch_bounds__(SOLVE ? SC_SOLVE_THREADS : IP_THREADS)
+__global__ void __maxnreg__(40)
     electron_scatter_kernel(const InplacePlanes pl, const CollList list, const float *__restrict__ cs,
                             uint32_t *count, uint32_t *ticket, uint32_t *n_e, uint32_t *n_i,
                             const __grid_constant__ cudapic_grid g, float *dens_e, float *dens_i,
