@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(IP_THREADS)
 // check_collisions_i / collision_i (Rust-CUDA/src/main.rs:1167-1292) of every
 // discharge, in place.  Plain coalesced loads; colliders go to warp-private
 // queues (slot and RNG state before the test) drained 32 at a time, as in
-// the resident-table kernel of kernels_mcc.cu, with each discharge's table
+// the streaming kernel of kernels_mcc.cu, with each discharge's table
 // read from global memory.
 constexpr int BC_U = 2;
 constexpr int BC_QCAP = 32 + 32 * BC_U;

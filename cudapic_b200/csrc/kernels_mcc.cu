@@ -12,17 +12,17 @@
 // B200 design: HBM-bound streaming (28 B read + 16 B RNG written per
 // particle; velocities written only by colliders, ~0.5 % of electrons per
 // step at the reference conditions).  Two kernels share the physics:
-//  * resident-table kernel (default, cudapic_tuning.mcc_variant = 1): one
-//    1024-thread CTA per SM keeps the first 32768 entries of sigma_tot in
-//    shared memory, every thread issues the loads of two particles before
-//    computing, and colliders go to warp-private queues drained 32 at a
+//  * streaming kernel (default, cudapic_tuning.mcc_variant = 1): one
+//    1024-thread CTA per SM, 16-byte loads, a certain rejection that needs no
+//    table; what it leaves open goes to warp-private queues drained 32 at a
 //    time -- no block barrier in the main loop;
 //  * bulk-copy kernel (mcc_variant = 2): tiles of the seven SoA arrays staged
-//    by cp.async.bulk on mbarriers, a CTA-wide collider queue.
+//    by cp.async.bulk on mbarriers, the full test on every particle (its
+//    provably exact fast reject skips exp() for almost all), a CTA-wide
+//    collider queue.
 // Common to both:
-//  * the collision test of every particle is uniform work; the provably
-//    exact fast reject skips exp() for almost all of them; non-colliders
-//    store their advanced RNG state (coalesced);
+//  * particles that the test rejects store their advanced RNG state
+//    (coalesced);
 //  * a collider keeps its slot and its RNG state before the test; the drain
 //    re-runs the deterministic test and scatters it on a full warp (one
 //    collider per lane) instead of one lane in 32;
@@ -34,6 +34,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "mcc.cuh"
+#include "step.cuh"
 #include "tma.cuh"
 
 namespace cudapic {
@@ -189,66 +190,136 @@ __global__ void __launch_bounds__(MCC_THREADS, 4)
     if (s_q > 0) drain();
 }
 
-// ------------------------------------------------------------------ resident-table kernels
+// ------------------------------------------------------------------ streaming kernel
 //
-// One 1024-thread CTA per SM, no bulk copies and no block barrier in the
-// main loop:
-//  * the first MR_RESIDENT entries of sigma_tot (energies below 32.768 eV,
-//    where almost every particle sits) are copied into shared memory once
-//    per launch; the collision-frequency gather becomes a shared load
-//    (higher energies still read the global table);
-//  * each thread issues the 7 loads of MR_U particles before any compute;
-//  * colliders go to a queue private to their warp (slot and RNG state
-//    before the test); whenever it holds 32 the warp drains 32 of them, one
-//    per lane -- only __syncwarp, no block-wide synchronisation.
-// Plain loads: no alignment requirement on any pointer.
+// One 1024-thread CTA per SM, no bulk copies and no block barrier in the main
+// loop; a warp takes tiles of 128 particles, four consecutive ones per lane
+// (16-byte loads where the planes are aligned and the group whole):
+//  * the certain rejection decides for nearly every particle without the
+//    table, a square root, a division or the target atom: electrons by
+//    may_collide's bound (step.cuh), ions by ion_collides' bound with the
+//    square root taken out (ion_surely_passes).  Both need the largest entry
+//    of the table the particle can meet: given by the caller (the bounded ion
+//    entry, the drivers), or found here, over the first MS_TABLE entries, by
+//    the CTAs of a cluster (half of the entries each, while the first
+//    tiles are on their way into L2); particles that
+//    could meet a higher entry's energy are not decided by it;
+//  * undecided particles go to a queue private to their warp (slot and RNG
+//    state before the test); whenever it holds 32 the warp takes 32 of them,
+//    one per lane, through the full test and, colliding, the scattering --
+//    only __syncwarp, no block-wide synchronisation.
+// Bound by memory (44 B per particle).  With the first 32768 entries copied to
+// every SM's shared memory and the full test on every particle (128 KB per
+// CTA and launch, scalar loads, a square root and a division each) 2 000 001
+// electrons took 30.3 us, now 25.5; 4 194 304 ions 49.4, now 40.1 (bounded); 1000
+// of either 8.0, now 6.7 and 4.7 (kernel alone).  Prefetching every tile and not
+// only the first into L2 gave nothing more.
 
-constexpr int MR_THREADS = 1024;
-constexpr int MR_WARPS = MR_THREADS / 32;
-constexpr int MR_U = 2;                        // particles per thread and iteration
-constexpr uint32_t MR_RESIDENT = 32768;        // sigma_tot entries kept in shared memory
-constexpr int MR_QCAP = 32 + 32 * MR_U;        // a warp drains at 32; one iteration adds <= 64
-constexpr size_t MR_SMEM = MR_RESIDENT * sizeof(float) + (size_t)MR_WARPS * 5 * MR_QCAP * sizeof(uint32_t);
+constexpr int MS_THREADS = 1024;
+constexpr int MS_WARPS = MS_THREADS / 32;
+constexpr int MS_ROW = 4;                       // particles per lane and tile
+constexpr int MS_TILE = 32 * MS_ROW;
+constexpr int MS_QCAP = 32 + MS_TILE;           // a warp drains at 32; one tile adds <= 128
+constexpr size_t MS_SMEM = (size_t)MS_WARPS * 5 * MS_QCAP * sizeof(uint32_t);
+constexpr int MS_CLUSTER = 2;                   // the largest that still reaches every SM (4 leaves some idle)
+constexpr uint32_t MS_TABLE = 32768;            // entries whose maximum a launch looks for
+constexpr float MS_TABLE_EV = 32.7f;            // energies below have an index below MS_TABLE
 
-template <bool ION, bool EVENTS>
-__global__ void __launch_bounds__(MR_THREADS, 1)
-    check_collisions_resident_kernel(const float *__restrict__ sigma_tot, const float *__restrict__ cs,
-                                     const uint32_t *__restrict__ active, float *x, float *vx, float *vy,
-                                     float *vz, uint32_t *rng0, uint32_t *rng1, uint32_t *rng2, uint32_t *rng3,
-                                     float *ix, float *ivx, float *ivy, float *ivz, uint32_t *alive_e,
-                                     uint32_t *alive_i, uint8_t *events, const __grid_constant__ cudapic_grid g,
-                                     float *dep_e, float *dep_i, unsigned long long *coll, float ion_k) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    float *tab = reinterpret_cast<float *>(smem);
+// True when the ion certainly does not collide, u the test draw (the fifth):
+// ion_collides decides so for u >= k (|v| + 9.2 sigma) + 6e-7.  Without the
+// root: with c >= 9.2 sigma k + 6.5e-7 and k2 >= k^2 (1 + 1e-4), y = fl(u - c)
+// >= 0 and fl(y y) >= fl(k2 v2) give y >= k |v| (each rounding is within
+// 2^-24 relative), hence u >= k |v| + c - 2^-24 > k (|v| + 9.2 sigma) + 5.8e-7,
+// which exceeds the computed collision probability (at most k (|v| + 9.2
+// sigma) + 3.1e-7).  NaN or infinite constants decide nothing.
+__device__ __forceinline__ bool ion_surely_passes(float u, float v2, float k2, float c) {
+    const float y = u - c;
+    return y >= 0.0f && y * y >= k2 * v2;
+}
+
+template <bool ION, bool EVENTS, bool BOUNDED>
+__global__ void __launch_bounds__(MS_THREADS, 1)
+    check_collisions_stream_kernel(const float *__restrict__ sigma_tot, const float *__restrict__ cs,
+                                   const uint32_t *__restrict__ active, float *x, float *vx, float *vy, float *vz,
+                                   uint32_t *rng0, uint32_t *rng1, uint32_t *rng2, uint32_t *rng3, float *ix,
+                                   float *ivx, float *ivy, float *ivz, uint32_t *alive_e, uint32_t *alive_i,
+                                   uint8_t *events, const __grid_constant__ cudapic_grid g, int vec, float *dep_e,
+                                   float *dep_i, unsigned long long *coll, float ion_k) {
+    extern __shared__ __align__(16) uint32_t ms_smem[];
+    __shared__ uint32_t s_max[MS_WARPS], s_top;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    uint32_t *wq = reinterpret_cast<uint32_t *>(tab + MR_RESIDENT) + (size_t)warp * 5 * MR_QCAP;  // [5][QCAP]
+    uint32_t *wq = ms_smem + (size_t)warp * 5 * MS_QCAP;  // [5][QCAP]
     const unsigned lt = lanemask_lt();
-
-    // the table is read before the wait: under PDL (the driver) it was
-    // written when the state was created, long before any dependent grid
-    for (uint32_t k = tid; k < MR_RESIDENT; k += MR_THREADS) tab[k] = __ldg(sigma_tot + k);
-    __syncthreads();
+    const float dt = ION ? g.dt_i : g.dt_e;
     grid_dep_wait();
-    const ResidentTable table{sigma_tot, tab, MR_RESIDENT};
     const uint32_t n = load_count(active, g.capacity, g.dev_err);
 
+    // largest energy-indexed entry the certain rejection may assume, and the
+    // largest v.v it then holds for
+    float k = ion_k;  // BOUNDED: max(sigma_tot) dt, rounded up
+    float v2_max = INFINITY;
+    if (!BOUNDED) {
+        const uint32_t j = (blockIdx.x + (uint32_t)warp * gridDim.x) * MS_TILE + (uint32_t)lane * MS_ROW;
+        if (j < n && (lane & 1) == 0) {  // one request per 32-byte sector of the warp's first tile
+            for (const void *p : {(const void *)(vx + j), (const void *)(vy + j), (const void *)(vz + j),
+                                  (const void *)(rng0 + j), (const void *)(rng1 + j), (const void *)(rng2 + j),
+                                  (const void *)(rng3 + j)})
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+        }
+        cg::cluster_group cluster = cg::this_cluster();
+        constexpr uint32_t part = MS_TABLE / MS_CLUSTER;
+        const float *mine = sigma_tot + cluster.block_rank() * part;
+        // entries compared as bit patterns: for non-negative floats their
+        // order; a negative or NaN entry makes a bound that decides nothing
+        uint32_t top = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < part / MS_THREADS; ++q) top = max(top, __float_as_uint(__ldg(mine + q * MS_THREADS + tid)));
+        top = __reduce_max_sync(0xffffffffu, top);
+        if (lane == 0) s_max[warp] = top;
+        __syncthreads();
+        if (warp == 0) {
+            top = __reduce_max_sync(0xffffffffu, s_max[lane]);
+            if (lane == 0) s_top = top;
+        }
+        cluster.sync();
+        top = __reduce_max_sync(0xffffffffu, lane < MS_CLUSTER ? *cluster.map_shared_rank(&s_top, lane) : 0u);
+        cluster.sync();  // no CTA leaves while its maximum is read
+        const float sigma_max = __uint_as_float(top);
+        k = ION ? sigma_max * dt * 1.00001f : sigma_max * dt;
+        if (ION) {  // |g| <= |v| + 9.2 sigma for every target atom: its energy below MS_TABLE_EV
+            const float v_max = sqrtf(MS_TABLE_EV / g.half_mu_over_e) - 9.21f * g.normal_range;
+            v2_max = v_max > 0.0f ? v_max * v_max * 0.9999f : -1.0f;
+        } else {
+            v2_max = MS_TABLE_EV / g.half_me_over_e;
+        }
+    }
+    const float k2 = k * k * 1.0001f;                                       // the bound on (nu dt)^2 / v.v
+    const float c = fmaf(k, 9.2f * g.normal_range, 6.5e-7f) * 1.000001f;    // ions: beside it
+    const GlobalTable table{sigma_tot};
+    // the four particles of a lane: neighbours for the vector loads, else 32
+    // apart, so that the scalar loads of a warp meet
+    const uint32_t di = vec ? 1u : 32u;
+
     auto drain = [&](uint32_t first, uint32_t count) {  // lanes < count take entries first + lane
-        if (coll && lane == 0) atomicAdd(coll, (unsigned long long)count);  // collision events (measurement)
+        bool hit = false;
         if ((uint32_t)lane < count) {
             const uint32_t q = first + lane;
-            const uint32_t i = wq[0 * MR_QCAP + q];
-            Xoshiro128p rs{wq[1 * MR_QCAP + q], wq[2 * MR_QCAP + q], wq[3 * MR_QCAP + q], wq[4 * MR_QCAP + q]};
+            const uint32_t i = wq[0 * MS_QCAP + q];
+            Xoshiro128p rs{wq[1 * MS_QCAP + q], wq[2 * MS_QCAP + q], wq[3 * MS_QCAP + q], wq[4 * MS_QCAP + q]};
             const float vxi = vx[i], vyi = vy[i], vzi = vz[i];
-            uint32_t ev;
+            uint32_t ev = 0;
             if (ION) {
                 const IonTest t = test_ion(vxi, vyi, vzi, rs, table, g);
-                ev = collide_ion(i, t.idx, vxi, vyi, vzi, t.vxa, t.vya, t.vza, rs, cs, vx, vy, vz, g);
+                hit = t.collide;
+                if (hit) ev = collide_ion(i, t.idx, vxi, vyi, vzi, t.vxa, t.vya, t.vza, rs, cs, vx, vy, vz, g);
             } else {
                 const Test t = test_electron(vxi, vyi, vzi, rs, table, g);
-                ev = collide_electron(0u, i, t.idx, vxi, vyi, vzi, rs, cs, x, vx, vy, vz, ix, ivx, ivy, ivz, alive_e,
-                                      alive_i, g, dep_e, dep_i);
+                hit = t.collide;
+                if (hit)
+                    ev = collide_electron(0u, i, t.idx, vxi, vyi, vzi, rs, cs, x, vx, vy, vz, ix, ivx, ivy, ivz, alive_e,
+                                          alive_i, g, dep_e, dep_i);
             }
             rng0[i] = rs.s0;
             rng1[i] = rs.s1;
@@ -256,60 +327,120 @@ __global__ void __launch_bounds__(MR_THREADS, 1)
             rng3[i] = rs.s3;
             if (EVENTS) events[i] = (uint8_t)ev;
         }
+        if (coll) {  // collision events (measurement)
+            const unsigned hits = __ballot_sync(0xffffffffu, hit);
+            if (lane == 0 && hits) atomicAdd(coll, (unsigned long long)__popc(hits));
+        }
         __syncwarp();
     };
 
     uint32_t qn = 0;  // entries in this warp's queue (warp-uniform)
-    const uint32_t step = gridDim.x * (uint32_t)(MR_THREADS * MR_U);
-    for (uint32_t base = blockIdx.x * (uint32_t)(MR_THREADS * MR_U); base < n; base += step) {
-        uint32_t s[MR_U][4];
-        float v[MR_U][3];
+    // tile t to CTA t mod gridDim: every SM gets the same number to within one
+    const uint32_t tiles = (uint32_t)(((uint64_t)n + MS_TILE - 1) / MS_TILE);
+    for (uint32_t t = blockIdx.x + (uint32_t)warp * gridDim.x; t < tiles; t += gridDim.x * MS_WARPS) {
+        const uint32_t i0 = t * MS_TILE + (uint32_t)lane * (vec ? MS_ROW : 1u);
+        const bool whole = vec && n - min(n, i0) >= MS_ROW;
+        uint32_t s[4][MS_ROW];
+        float v[3][MS_ROW];
+        if (whole) {
+            const float4 a = *reinterpret_cast<const float4 *>(vx + i0), b = *reinterpret_cast<const float4 *>(vy + i0);
+            const float4 d = *reinterpret_cast<const float4 *>(vz + i0);
+            const uint4 e = *reinterpret_cast<const uint4 *>(rng0 + i0), f = *reinterpret_cast<const uint4 *>(rng1 + i0);
+            const uint4 h = *reinterpret_cast<const uint4 *>(rng2 + i0), w = *reinterpret_cast<const uint4 *>(rng3 + i0);
+            v[0][0] = a.x, v[0][1] = a.y, v[0][2] = a.z, v[0][3] = a.w;
+            v[1][0] = b.x, v[1][1] = b.y, v[1][2] = b.z, v[1][3] = b.w;
+            v[2][0] = d.x, v[2][1] = d.y, v[2][2] = d.z, v[2][3] = d.w;
+            s[0][0] = e.x, s[0][1] = e.y, s[0][2] = e.z, s[0][3] = e.w;
+            s[1][0] = f.x, s[1][1] = f.y, s[1][2] = f.z, s[1][3] = f.w;
+            s[2][0] = h.x, s[2][1] = h.y, s[2][2] = h.z, s[2][3] = h.w;
+            s[3][0] = w.x, s[3][1] = w.y, s[3][2] = w.z, s[3][3] = w.w;
+        } else {
 #pragma unroll
-        for (int u = 0; u < MR_U; ++u) {
-            const uint32_t i = base + (uint32_t)u * MR_THREADS + tid;
-            if (i < n) {
-                s[u][0] = rng0[i];
-                s[u][1] = rng1[i];
-                s[u][2] = rng2[i];
-                s[u][3] = rng3[i];
-                v[u][0] = vx[i];
-                v[u][1] = vy[i];
-                v[u][2] = vz[i];
+            for (uint32_t u = 0; u < MS_ROW; ++u) {
+                const bool in = i0 + u * di < n;
+                v[0][u] = in ? vx[i0 + u * di] : 0.0f;
+                v[1][u] = in ? vy[i0 + u * di] : 0.0f;
+                v[2][u] = in ? vz[i0 + u * di] : 0.0f;
+                s[0][u] = in ? rng0[i0 + u * di] : 0u;
+                s[1][u] = in ? rng1[i0 + u * di] : 0u;
+                s[2][u] = in ? rng2[i0 + u * di] : 0u;
+                s[3][u] = in ? rng3[i0 + u * di] : 0u;
             }
         }
+        uint32_t open = 0;  // bit u: not decided by the bound (its state stays before the test)
 #pragma unroll
-        for (int u = 0; u < MR_U; ++u) {
-            const uint32_t i = base + (uint32_t)u * MR_THREADS + tid;
-            bool collide = false;
-            if (i < n) {
-                Xoshiro128p rs{s[u][0], s[u][1], s[u][2], s[u][3]};
-                if (ION) collide = ion_collides(v[u][0], v[u][1], v[u][2], rs, table, g, ion_k);
-                else collide = test_electron(v[u][0], v[u][1], v[u][2], rs, table, g).collide;
-                if (!collide) {
-                    rng0[i] = rs.s0;
-                    rng1[i] = rs.s1;
-                    rng2[i] = rs.s2;
-                    rng3[i] = rs.s3;
-                    if (EVENTS) events[i] = 0;
+        for (int u = 0; u < MS_ROW; ++u) {
+            const float v2 = v[0][u] * v[0][u] + v[1][u] * v[1][u] + v[2][u] * v[2][u];
+            Xoshiro128p rs{s[0][u], s[1][u], s[2][u], s[3][u]};
+            bool passes;
+            if (ION) {
+                rs.next();  // the target atom's four draws
+                rs.next();
+                rs.next();
+                rs.next();
+                passes = ion_surely_passes(rs.uniform(), v2, k2, c);
+            } else {
+                passes = !may_collide(rs.uniform(), v2, k2);
+            }
+            if (passes && (BOUNDED || v2 < v2_max)) {
+                s[0][u] = rs.s0;
+                s[1][u] = rs.s1;
+                s[2][u] = rs.s2;
+                s[3][u] = rs.s3;
+            } else if (i0 + (uint32_t)u * di < n) {
+                open |= 1u << u;
+            }
+        }
+        if (whole) {  // open ones keep their state until their drain
+            *reinterpret_cast<uint4 *>(rng0 + i0) = make_uint4(s[0][0], s[0][1], s[0][2], s[0][3]);
+            *reinterpret_cast<uint4 *>(rng1 + i0) = make_uint4(s[1][0], s[1][1], s[1][2], s[1][3]);
+            *reinterpret_cast<uint4 *>(rng2 + i0) = make_uint4(s[2][0], s[2][1], s[2][2], s[2][3]);
+            *reinterpret_cast<uint4 *>(rng3 + i0) = make_uint4(s[3][0], s[3][1], s[3][2], s[3][3]);
+        } else {
+#pragma unroll
+            for (uint32_t u = 0; u < MS_ROW; ++u) {
+                if (i0 + u * di >= n) continue;
+                rng0[i0 + u * di] = s[0][u];
+                rng1[i0 + u * di] = s[1][u];
+                rng2[i0 + u * di] = s[2][u];
+                rng3[i0 + u * di] = s[3][u];
+            }
+        }
+        if (EVENTS) {
+#pragma unroll
+            for (uint32_t u = 0; u < MS_ROW; ++u)
+                if (i0 + u * di < n) events[i0 + u * di] = 0;  // an open one's own event follows with its drain
+        }
+        if (__ballot_sync(0xffffffffu, open != 0)) {
+#pragma unroll
+            for (int u = 0; u < MS_ROW; ++u) {
+                const unsigned m = __ballot_sync(0xffffffffu, open >> u & 1u);
+                if (open >> u & 1u) {
+                    const uint32_t q = qn + __popc(m & lt);
+                    wq[0 * MS_QCAP + q] = i0 + (uint32_t)u * di;
+                    wq[1 * MS_QCAP + q] = s[0][u];
+                    wq[2 * MS_QCAP + q] = s[1][u];
+                    wq[3 * MS_QCAP + q] = s[2][u];
+                    wq[4 * MS_QCAP + q] = s[3][u];
+                    if (!ION) {  // the drain's gathers, fetched together instead of one after the other
+                        const float v2 = v[0][u] * v[0][u] + v[1][u] * v[1][u] + v[2][u] * v[2][u];
+                        const uint32_t e = energy_index(g.half_me_over_e * v2);
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(sigma_tot + e));
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(cs + e));
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(cs + CS_RANGES + e));
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(cs + 2 * CS_RANGES + e));
+                    }
                 }
+                qn += __popc(m);
             }
-            const unsigned m = __ballot_sync(0xffffffffu, collide);
-            if (collide) {
-                const uint32_t q = qn + __popc(m & lt);
-                wq[0 * MR_QCAP + q] = i;
-                wq[1 * MR_QCAP + q] = s[u][0];
-                wq[2 * MR_QCAP + q] = s[u][1];
-                wq[3 * MR_QCAP + q] = s[u][2];
-                wq[4 * MR_QCAP + q] = s[u][3];
+            __syncwarp();
+            while (qn >= 32) {  // full-warp drains from the top of the queue
+                qn -= 32;
+                drain(qn, 32);
             }
-            qn += __popc(m);
-        }
-        __syncwarp();
-        while (qn >= 32) {  // full-warp drains from the top of the queue
-            qn -= 32;
-            drain(qn, 32);
         }
     }
+    __syncwarp();
     if (qn) drain(0, qn);
 }
 
@@ -424,23 +555,59 @@ int launch_tma(const float *sigma_tot, const float *cs, const uint32_t *active, 
                          alive_i, events, g, stages, dep_e, dep_i, coll, ion_k);
 }
 
-template <bool ION, bool EVENTS>
-int launch_resident(const float *sigma_tot, const float *cs, const uint32_t *active, float *x, float *vx, float *vy,
+template <bool ION, bool EVENTS, bool BOUNDED>
+int launch_stream_t(const float *sigma_tot, const float *cs, const uint32_t *active, float *x, float *vx, float *vy,
                     float *vz, uint32_t *r0, uint32_t *r1, uint32_t *r2, uint32_t *r3, float *ix, float *ivx,
                     float *ivy, float *ivz, uint32_t *alive_e, uint32_t *alive_i, uint8_t *events,
                     const cudapic_grid &g, cudaStream_t stream, float *dep_e, float *dep_i,
                     unsigned long long *coll, float ion_k) {
-    auto kern = check_collisions_resident_kernel<ION, EVENTS>;
-    if (MR_SMEM > (size_t)max_smem_optin()) return fail(CUDAPIC_ERR_NOT_SUPPORTED, "check_collisions: shared memory");
-    CUDAPIC_CHECK(kernel_smem((const void *)kern, MR_SMEM, "check_collisions"));
-    const uint64_t chunks = ((uint64_t)g.capacity + MR_THREADS * MR_U - 1) / (MR_THREADS * MR_U);
-    return launch_kernel(ION ? "check_collisions_i" : "check_collisions_e", kern, dim3(persistent_grid(1, chunks)),
-                         dim3(MR_THREADS), MR_SMEM, stream, sigma_tot, cs, active, x, vx, vy, vz, r0, r1, r2, r3, ix,
-                         ivx, ivy, ivz, alive_e, alive_i, events, g, dep_e, dep_i, coll, ion_k);
+    auto kern = check_collisions_stream_kernel<ION, EVENTS, BOUNDED>;
+    const char *name = ION ? "check_collisions_i" : "check_collisions_e";
+    CUDAPIC_CHECK(kernel_smem((const void *)kern, MS_SMEM, name));
+    bool vec = true;
+    for (const void *p : {(const void *)vx, (const void *)vy, (const void *)vz, (const void *)r0, (const void *)r1,
+                          (const void *)r2, (const void *)r3})
+        vec = vec && aligned16(p);
+    constexpr unsigned cl = BOUNDED ? 1 : MS_CLUSTER;  // the unbounded kernel finds its bound in clusters
+    unsigned grid = persistent_grid(1, ((uint64_t)g.capacity + MS_TILE - 1) / MS_TILE);
+    grid = grid / cl * cl ? grid / cl * cl : cl;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(MS_THREADS);
+    cfg.dynamicSmemBytes = MS_SMEM;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    if (!BOUNDED) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cl;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
+    if (pdl_enabled()) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+        ++cfg.numAttrs;
+    }
+    CUDAPIC_CHECK(check_cuda(cudaLaunchKernelEx(&cfg, kern, sigma_tot, cs, active, x, vx, vy, vz, r0, r1, r2, r3, ix, ivx,
+                                                ivy, ivz, alive_e, alive_i, events, g, (int)vec, dep_e, dep_i, coll,
+                                                ion_k), name));
+    return check_launch(name);
+}
+
+// A finite ion_k is the caller's bound for the ion test; electrons and ions
+// without one find theirs in the launch.
+template <bool ION, bool EVENTS, typename... Args>
+int launch_stream(float ion_k, Args... args) {
+    if constexpr (ION) {
+        if (ion_k < INFINITY) return launch_stream_t<ION, EVENTS, true>(args..., ion_k);
+    }
+    return launch_stream_t<ION, EVENTS, false>(args..., ion_k);
 }
 
 // Variant choice: the bulk-copy kernel needs 16-byte aligned planes and a
-// capacity that is a multiple of 4; the resident-table kernel takes anything.
+// capacity that is a multiple of 4; the streaming kernel takes anything.
 template <bool ION>
 int launch_collisions(const float *sigma_tot, const float *cs, const uint32_t *active, float *x, float *vx,
                       float *vy, float *vz, uint32_t *r0, uint32_t *r1, uint32_t *r2, uint32_t *r3, float *ix,
@@ -456,10 +623,10 @@ int launch_collisions(const float *sigma_tot, const float *cs, const uint32_t *a
                                       alive_e, alive_i, nullptr, g, stream, dep_e, dep_i, coll, ion_k);
     }
     if (events)
-        return launch_resident<ION, true>(sigma_tot, cs, active, x, vx, vy, vz, r0, r1, r2, r3, ix, ivx, ivy, ivz,
-                                          alive_e, alive_i, events, g, stream, dep_e, dep_i, coll, ion_k);
-    return launch_resident<ION, false>(sigma_tot, cs, active, x, vx, vy, vz, r0, r1, r2, r3, ix, ivx, ivy, ivz,
-                                       alive_e, alive_i, nullptr, g, stream, dep_e, dep_i, coll, ion_k);
+        return launch_stream<ION, true>(ion_k, sigma_tot, cs, active, x, vx, vy, vz, r0, r1, r2, r3, ix, ivx, ivy, ivz,
+                                        alive_e, alive_i, events, g, stream, dep_e, dep_i, coll);
+    return launch_stream<ION, false>(ion_k, sigma_tot, cs, active, x, vx, vy, vz, r0, r1, r2, r3, ix, ivx, ivy, ivz,
+                                     alive_e, alive_i, (uint8_t *)nullptr, g, stream, dep_e, dep_i, coll);
 }
 
 }  // namespace

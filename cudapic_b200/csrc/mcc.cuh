@@ -121,19 +121,10 @@ struct Test {
     bool collide;
 };
 
-// sigma_tot lookups: straight from the global table (read-only path), or
-// from a shared-memory copy of its first `resident` entries.
+// sigma_tot lookups from the global table (read-only path).
 struct GlobalTable {
     const float *__restrict__ t;
     __device__ __forceinline__ float operator()(uint32_t idx) const { return __ldg(t + idx); }
-};
-struct ResidentTable {
-    const float *__restrict__ t;   // global table
-    const float *s;                // shared copy of t[0 .. resident)
-    uint32_t resident;
-    __device__ __forceinline__ float operator()(uint32_t idx) const {
-        return idx < resident ? s[idx] : __ldg(t + idx);
-    }
 };
 
 // Electron collision test, Rust-CUDA/src/main.rs:992-1012 (one draw).

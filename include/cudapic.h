@@ -139,7 +139,7 @@ typedef struct cudapic_tuning {
     int push_ctas_per_sm;
     int mcc_stages;           /* check_collisions_e/i pipeline depth: 2..4               */
     int mcc_ctas_per_sm;
-    int mcc_variant;          /* 1: shared-memory resident sigma table (any alignment),
+    int mcc_variant;          /* 1: streaming, certain rejection first (any alignment),
                                  2: bulk-copy staged tiles (16-byte aligned pointers)    */
     int step_stages;          /* fused electron step bulk-copy pipeline depth: 2..6      */
     int step_ctas_per_sm;

@@ -671,6 +671,36 @@ def test_check_collisions_i_bit_exact(cudapic, K, oracle, dev_tables, tables, n,
         assert np.array_equal(_read(d)[:n].view(np.uint32), h[:n].view(np.uint32))
 
 
+@pytest.mark.parametrize("species,bounded", [("e", False), ("i", False), ("i", True)])
+@pytest.mark.parametrize("n,shifted", [(3, ()), (127, ()), (128, ()), (129, (5,)), (4737, (0,)), (606_209, ()),
+                                       (606_207, (0, 1, 2, 3, 4, 5, 6))])
+def test_check_collisions_tile_edges(cudapic, K, oracle, dev_tables, tables, species, bounded, n, shifted):
+    """Around the tiles of 128 particles and one tile per warp of the grid, the
+    count the capacity itself (nothing may be read past it), any of the seven
+    planes off 16 bytes."""
+    cs, se, si = tables
+    dcs, dse, dsi = dev_tables
+    g = cudapic.grid_from_params(n_t=200, capacity=n)
+    ph = oracle.phys_from_params(n_t=200, capacity=n)
+    x, vx, vy, vz = _mcc_case(n, 20.0 if species == "e" else 2.0, n + 2, E_MASS if species == "e" else AR_MASS)
+    r_h = [np.asarray(p).copy() for p in oracle.seed_streams([n, 6, 7, 8], n)]
+    v_h = [vx.copy(), vy.copy(), vz.copy()]
+    planes = [_dev_layout(a, "unaligned" if k in shifted else "aligned") for k, a in enumerate(v_h + r_h)]
+    events = zeros(n, np.uint8)
+    if species == "e":
+        e_h, i_h = [x.copy()] + v_h, [np.zeros(n, np.float32) for _ in range(4)]
+        K.check_collisions_e(dse, dcs, counter(n), dev(x), *planes, *[zeros(n) for _ in range(4)], counter(n), counter(0),
+                             g, events=events)  # no room for spawned electrons
+        ev_ref, _, _, _ = oracle.check_collisions_e(se, cs, n, e_h, r_h, i_h, n, 0, ph)
+    else:
+        K.check_collisions_i(dsi, dcs, counter(n), *planes, g, events=events,
+                             sigma_max_i=float(si.max()) if bounded else None)
+        ev_ref = oracle.check_collisions_i(si, cs, n, v_h, r_h, ph)
+    assert np.array_equal(host(events), ev_ref)
+    for d, h in zip(planes, v_h + r_h):
+        assert np.array_equal(_read(d)[:n].view(np.uint32), h[:n].view(np.uint32))
+
+
 def test_spawn_capacity_is_enforced(cudapic, K, oracle, dev_tables, tables):
     """Ionization spawns beyond capacity are dropped and flagged, never
     written past the buffers (the reference writes unbounded)."""

@@ -60,3 +60,42 @@ def test_no_ion_above_the_bound_collides(cudapic, oracle, tables, n_t, temp, see
     assert np.any(events > 0)
     if n_t == 4000:  # the reference's time step: nearly every ion skips the target's transcendentals
         assert skipped.mean() > 0.9, skipped.mean()
+
+
+@pytest.mark.parametrize("n_t,temp,seed", [(4000, 0.03, 11), (4000, 2.0, 12), (200, 0.03, 13), (200, 20.0, 14),
+                                           (20, 2.0, 15), (20, 20.0, 16)])
+def test_bound_without_the_root_is_the_stricter_one(cudapic, oracle, tables, n_t, temp, seed):
+    """kernels_mcc.cu's ion_surely_passes: the bound with the square root
+    taken out.  Every draw it lets pass lies above the bound with the root, so
+    no such ion collides, and it still decides nearly every thermal ion."""
+    from cudapic_b200.workloads import steady_state
+    f = np.float32
+    cs, _, si = tables
+    n = 200_000
+    g = cudapic.grid_from_params(n_t=n_t, capacity=n)
+    ph = oracle.phys_from_params(n_t=n_t, capacity=n)
+    k = np.nextafter(f(float(si.max()) * float(g.dt_i) * (1.0 + 1e-5)), f(np.inf))
+    k2 = (k * k).astype(f) * f(1.0001)
+    c = f(np.float64(k) * np.float64(f(9.2) * f(g.normal_range)) + 6.5e-7) * f(1.000001)
+    _, vx, vy, vz = steady_state(n, AR_MASS, temp, seed=seed, edge_fraction=0.0)
+    v2 = (vx * vx + vy * vy + vz * vz).astype(f)
+
+    def passes(u):
+        y = (u - c).astype(f)
+        return (y >= 0) & ((y * y).astype(f) >= (k2 * v2).astype(f))
+
+    rng = [np.asarray(p).copy() for p in oracle.seed_streams([seed, 7, 11, 13], n)]
+    s = [p.copy() for p in rng]
+    for _ in range(4):
+        _next(s)
+    u = _uniform(_next(s))
+    events = oracle.check_collisions_i(si, cs, n, [vx.copy(), vy.copy(), vz.copy()], [p.copy() for p in rng], ph)
+    assert not np.any(events[passes(u)])
+    b = _bound(k, vx, vy, vz, g.normal_range)
+    assert np.all(u[passes(u)] >= b[passes(u)])
+    # draws within a few ulp and within 1e-4 of the bound, where the two could differ
+    for near in [b + f(d) for d in (-2e-7, -6e-8, 0.0, 6e-8, 1.2e-7, 1e-6, 1e-5)] + [(b * f(r)).astype(f) for r in (0.9999, 1.0001)]:
+        near = near.astype(f)
+        assert np.all(near[passes(near)] >= b[passes(near)])
+    if n_t == 4000:
+        assert passes(u).mean() > 0.9
