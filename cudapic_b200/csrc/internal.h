@@ -196,14 +196,15 @@ int rng_sidecar_read(const char *path, uint32_t capacity, std::vector<uint32_t> 
 // colliders are recorded in `list` / *count -- and the scatter pass over the
 // records (spawns appended at *n_e and *n_i; its last CTA adds the
 // collision count to *coll and clears *count and *ticket).  spawn_from (may
-// be null): receives the slot count the stream pass saw.
+// be null): receives the slot count the stream pass saw.  reverse: the slots
+// from the last to the first.
 struct InplacePlanes;
 struct CollList;
 int launch_electron_inplace(const InplacePlanes &pl, const float *efield, const float *sigma_tot_e, const float *cs,
                             float sigma_max, const uint32_t *n_active, const CollList &list, uint32_t *count,
                             float *dens_e,
                             const cudapic_grid &g, cudaStream_t stream, cudapic_wall_counters *wall,
-                            uint32_t *spawn_from);
+                            uint32_t *spawn_from, bool reverse = false);
 // The next step's Poisson solve (launch_poisson's arguments), run by the
 // last CTA of the scatter pass once every CTA has added its spawns.
 struct PoissonAhead {

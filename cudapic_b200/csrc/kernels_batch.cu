@@ -213,7 +213,7 @@ template <bool MEAS>
 __global__ void __launch_bounds__(IP_THREADS, 4)
     batch_inplace_kernel(const __grid_constant__ InplacePlanes pl, const __grid_constant__ CollList list,
                          const BatchDisc *__restrict__ desc, const uint32_t *__restrict__ counts, uint32_t D,
-                         int dens_role, uint32_t ef_pad, int copies, uint32_t epoch, uint32_t pf) {
+                         int dens_role, uint32_t ef_pad, int copies, uint32_t epoch, uint32_t pf, int reverse) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint32_t wsum[ES_WARPS];
     __shared__ StepDisc s_dc;
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(IP_THREADS, 4)
                                 list.r0 + off,   list.r1 + off, list.r2 + off, list.r3 + off};
             uint32_t live = 0;
             inplace_segment<true, MEAS>(pl, s_dc, g, s_g, off, lo, hi, sm, copies, ef_pad, epoch, mine,
-                                        dcp<true>(s_dc.alive), live, pf);
+                                        dcp<true>(s_dc.alive), live, pf, rounds_of(lo, hi, 0u, 1u, reverse != 0));
             add_work(s_g.work, live);
         }
         d = lds_volatile(&s_d);
@@ -632,7 +632,8 @@ int launch_batch_inplace(const InplacePlanes &pl, const CollList &list, const Ba
     const uint32_t per_round = copies ? (uint32_t)((IP_WARPS + copies - 1) / copies) * 32u * IP_ROW : 1u;
     const uint32_t epoch = copies ? std::max(1u, DEP_MAX_PER_COPY / per_round) : 0xffffffffu;
     return launch_kernel("batch_inplace_electrons", kern, dim3(grid), dim3(IP_THREADS), bytes(), stream, pl, list,
-                         desc, counts, D, r.dens, ef_pad, copies, epoch, (uint32_t)std::max(t.inplace_prefetch, 0));
+                         desc, counts, D, r.dens, ef_pad, copies, epoch, (uint32_t)std::max(t.inplace_prefetch ? t.inplace_prefetch : 1, 0),
+                         r.dens);  // the role turns every step, and the direction with it
 }
 
 int launch_batch_scatter(const InplacePlanes &pl, const CollList &list, const BatchDisc *desc, uint32_t D,

@@ -148,7 +148,8 @@ typedef struct cudapic_tuning {
     int inplace_copies;       /* in-place electron step: fixed-point deposit histogram copies
                                  (1..8), -1: one f32 shared histogram                     */
     int inplace_prefetch;     /* in-place electron step: rounds of a CTA's slots prefetched
-                                 into L2 ahead of their loads (1..4), -1: none             */
+                                 into L2 ahead of their loads (1..4), -1: none, 0: none
+                                 for one discharge, 1 for a batch                          */
     int scatter_ctas_per_sm;  /* in-place electron step, scatter pass: CTAs per SM (1..8)   */
 } cudapic_tuning;
 

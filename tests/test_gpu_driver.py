@@ -97,6 +97,33 @@ def test_work_counter_counts_particle_steps(cudapic, cuda_device):
     st.close()
 
 
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 606_207, 606_208, 606_209, 1_212_417])
+def test_every_slot_is_pushed_once_in_either_direction(cudapic, cuda_device, n):
+    """Three steps, in place from the last slot to the first, from the first to
+    the last, and compacting, of electrons that neither meet nor move anything
+    (no gas, no charge, no voltage): x += vx dt in f32, three times, exactly.
+    Counts around the tiles of 1024 slots and one tile per CTA of 4 x 148."""
+    from cudapic_b200.sim import GpuSimState, ParticlesSoA
+    params = cudapic.default_params(capacity=max(40_000, (n + 7) // 4 * 4), voltage=0.0, pressure=1e-9, weight=1e-20)
+    rng = np.random.default_rng(n)
+    x = (0.025 * rng.uniform(0.2, 0.8, n)).astype(np.float32)
+    v = rng.normal(0.0, 3e5, (3, n)).astype(np.float32)
+    st = GpuSimState(params)
+    st.upload_electrons(ParticlesSoA(x, *v))
+    st.upload_ions(ParticlesSoA(x[:1], *(np.zeros(1, np.float32) for _ in range(3))))
+    st.seed()
+    st.run_steps(3)
+    p, m = st.download_electrons()
+    assert m == n and st.counts() == (n, 1) and st.device_error() == 0 and st.work() == 3 * n + 1
+    dt = np.float32(cudapic.grid_from_params(params).dt_e)
+    for _ in range(3):
+        x = x + v[0] * dt
+    key, ref = np.lexsort((p.vz, p.vy)), np.lexsort((v[2], v[1]))
+    for a, b in zip((p.x, p.vx, p.vy, p.vz), (x, *v)):
+        assert np.array_equal(a[key], b[ref])
+    st.close()
+
+
 def test_graph_replay_equals_direct_launch_statistics(cudapic, cuda_device):
     """run_steps(40) (one graph replay) and 40 x run_steps(1) (direct launches)
     enqueue the same sequence; with the same seeds and inputs the counts agree
