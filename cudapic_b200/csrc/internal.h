@@ -99,19 +99,32 @@ struct StepLink {
 };
 
 // Launchers used by both the drop-in entry points and the driver.
+// eepf (may be null): the previous step's EEPF samples, taken by further CTAs
+// of the launch (its efield must not be the field written here).
 // zero_a / zero_b (may be null): n_g-float buffers the kernel clears after
 // reading the densities (the driver's next-step density accumulators).
 // meas (cumul_e null: none): the grid quantities of a measured step -- the
 // time-averaged densities (cumul_i on ion steps only) and the XT column of
 // the step (xt may be null) -- added by the solve's own launch; needs a step
-// counter.
+// counter.  ef_keep (may be null): a second copy of the field.
 struct PoissonMeasure {
     double *cumul_e, *cumul_i, *xt;
     uint32_t n_xt;
+    float *ef_keep;
+};
+// One step's EEPF samples (eepf.cuh): the electrons after the step and the
+// field that pushed them; esum, ecount: the centre-energy sums (may be null).
+struct EepfSamples {
+    const float *x, *vx, *vy, *vz, *efield;
+    const uint32_t *active_e;
+    uint32_t *eepf;
+    double *esum;
+    unsigned long long *ecount;
 };
 int launch_poisson(const float *e_density, const float *i_density, float *pot, float *efield, float pot0,
                    const float *pot0_table, uint32_t *step_counter, const cudapic_grid &g, cudaStream_t stream,
-                   float *zero_a = nullptr, float *zero_b = nullptr, const PoissonMeasure &meas = PoissonMeasure{});
+                   float *zero_a = nullptr, float *zero_b = nullptr, const PoissonMeasure &meas = PoissonMeasure{},
+                   const EepfSamples *eepf = nullptr);
 // Adjoint of launch_poisson's solve and field in FP64 (kernels_poisson.cu):
 // eb (field adjoint, cleared) -> neb, nib_acc (density adjoints, the ion one
 // accumulated unless reset_acc) and vbar += cosv * (pot0 adjoint), for `obs`
@@ -162,9 +175,7 @@ int launch_collisions_i(const float *total_cs_i, const float *cs, const uint32_t
                         float ion_k = INFINITY);
 // The bound ion_k for a table whose largest entry is sigma_max_i.
 float ion_reject_k(float sigma_max_i, const cudapic_grid &g);
-int launch_eepf(const float *x, const float *vx, const float *vy, const float *vz, const float *efield,
-                const uint32_t *active_e, uint32_t *eepf, const cudapic_grid &g, cudaStream_t stream,
-                double *esum = nullptr, unsigned long long *ecount = nullptr);
+int launch_eepf(const EepfSamples &a, const cudapic_grid &g, cudaStream_t stream);
 
 // XT diagnostics (kernels_xt.cu): steps per column (eduPIC's N_BIN) and the
 // raw accumulators, each [n_g][n_xt] doubles, n_xt = N_T / XT_BIN.

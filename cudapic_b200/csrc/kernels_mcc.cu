@@ -32,6 +32,7 @@
 //    :1132-1149);
 //  * transcendentals from detmath.cuh (bit-reproducible, see there).
 #include "common.cuh"
+#include "eepf.cuh"
 #include "internal.h"
 #include "mcc.cuh"
 #include "step.cuh"
@@ -444,87 +445,12 @@ __global__ void __launch_bounds__(MS_THREADS, 1)
     if (qn) drain(0, qn);
 }
 
-// accumulate_eepf, Rust-CUDA/src/main.rs:1301-1339: per-block shared
-// histogram, one global atomic per non-empty bin and block.  Four consecutive
-// positions per thread and round (VEC: one 16-byte load; x must be aligned),
-// velocities only of the electrons in the window; the centre-energy sums are
-// reduced over the block before their two global atomics (one pair per warp
-// serialised thousands of atomics on two addresses): 400 000 electrons 9.5 us,
-// now 5.3 us.
+// accumulate_eepf as a launch of its own (eepf.cuh).
 constexpr int EEPF_THREADS = 512;
 
-template <bool VEC>
 __global__ void __launch_bounds__(EEPF_THREADS)
-    accumulate_eepf_kernel(const float *__restrict__ x, const float *__restrict__ vx, const float *__restrict__ vy,
-                           const float *__restrict__ vz, const float *__restrict__ efield,
-                           const uint32_t *__restrict__ active_e, uint32_t *__restrict__ eepf,
-                           const __grid_constant__ cudapic_grid g, double *esum, unsigned long long *ecount) {
-    __shared__ uint32_t h[N_EEPF];
-    __shared__ double s_sum[EEPF_THREADS / 32];
-    __shared__ uint32_t s_cnt[EEPF_THREADS / 32];
-    for (uint32_t k = threadIdx.x; k < N_EEPF; k += EEPF_THREADS) h[k] = 0;
-    __syncthreads();
-    grid_dep_wait();
-    const uint32_t n = load_count(active_e, g.capacity, g.dev_err);
-    double e_sum = 0.0;
-    uint32_t e_cnt = 0;
-    auto sample = [&](uint32_t i, float xi) {
-        if (xi <= g.min_x || xi >= g.max_x) return;
-        const float pos = xi * g.inv_dx;
-        const int p = cell_of(pos, g.n_g);
-        const float c2 = pos - (float)p;
-        const float e_x = (1.0f - c2) * __ldg(efield + p) + c2 * __ldg(efield + p + 1);
-        const float mvx = vx[i] - 0.5f * e_x * g.eepf_half_kick;
-        const float vyi = vy[i], vzi = vz[i];
-        const float v2 = mvx * mvx + vyi * vyi + vzi * vzi;
-        const float energy = g.half_me_over_e * v2;
-        const float binf = energy / DE_EEPF_F;
-        if (binf < (float)N_EEPF) atomicAdd(&h[(uint32_t)binf], 1u);
-        e_sum += (double)energy;
-        ++e_cnt;
-    };
-    const uint64_t stride = (uint64_t)gridDim.x * EEPF_THREADS;
-    for (uint64_t j = (uint64_t)blockIdx.x * EEPF_THREADS + threadIdx.x; 4u * j < n; j += stride) {
-        const uint32_t i0 = (uint32_t)(4u * j);
-        float xs[4];
-        if (VEC && i0 + 4u <= n) {
-            const float4 X = *reinterpret_cast<const float4 *>(x + i0);
-            xs[0] = X.x;
-            xs[1] = X.y;
-            xs[2] = X.z;
-            xs[3] = X.w;
-        } else {
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u) xs[u] = i0 + u < n ? x[i0 + u] : g.min_x;  // min_x: not sampled
-        }
-#pragma unroll
-        for (uint32_t u = 0; u < 4; ++u) sample(i0 + u, xs[u]);
-    }
-    if (esum) {  // mean energy of the sampled electrons (the report's centre energy)
-        for (int o = 16; o > 0; o >>= 1) {
-            e_sum += __shfl_down_sync(0xffffffffu, e_sum, o);
-            e_cnt += __shfl_down_sync(0xffffffffu, e_cnt, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            s_sum[threadIdx.x >> 5] = e_sum;
-            s_cnt[threadIdx.x >> 5] = e_cnt;
-        }
-    }
-    __syncthreads();
-    if (esum && threadIdx.x == 0) {
-        unsigned long long c = 0;
-        e_sum = 0.0;
-        for (int w = 0; w < EEPF_THREADS / 32; ++w) {
-            e_sum += s_sum[w];
-            c += s_cnt[w];
-        }
-        if (c) {
-            atomicAdd(esum, e_sum);
-            atomicAdd(ecount, c);
-        }
-    }
-    for (uint32_t k = threadIdx.x; k < N_EEPF; k += EEPF_THREADS)
-        if (h[k]) atomicAdd(&eepf[k], h[k]);
+    accumulate_eepf_kernel(const EepfSamples a, const __grid_constant__ cudapic_grid g, int vec) {
+    eepf_accumulate(a, g, vec != 0, blockIdx.x, gridDim.x);
 }
 
 namespace {
@@ -654,13 +580,10 @@ float ion_reject_k(float sigma_max_i, const cudapic_grid &g) {
     return std::nextafter((float)k, INFINITY);
 }
 
-int launch_eepf(const float *x, const float *vx, const float *vy, const float *vz, const float *efield,
-                const uint32_t *active_e, uint32_t *eepf, const cudapic_grid &g, cudaStream_t stream,
-                double *esum, unsigned long long *ecount) {
+int launch_eepf(const EepfSamples &a, const cudapic_grid &g, cudaStream_t stream) {
     const unsigned grid = persistent_grid(2, ((uint64_t)g.capacity + 4 * EEPF_THREADS - 1) / (4 * EEPF_THREADS));
-    return launch_kernel("accumulate_eepf", aligned16(x) ? accumulate_eepf_kernel<true> : accumulate_eepf_kernel<false>,
-                         dim3(grid), dim3(EEPF_THREADS), 0, stream, x, vx, vy, vz, efield, active_e, eepf, g, esum,
-                         ecount);
+    return launch_kernel("accumulate_eepf", accumulate_eepf_kernel, dim3(grid), dim3(EEPF_THREADS), 0, stream, a, g,
+                         (int)aligned16(a.x));
 }
 
 }  // namespace cudapic
@@ -750,5 +673,6 @@ extern "C" int cudapic_accumulate_eepf(const float *x, const float *vx, const fl
                                        const cudapic_grid *grid, cudapic_stream_t stream) {
     CUDAPIC_CHECK(validate_grid(grid));
     CUDAPIC_REQUIRE(x && vx && vy && vz && efield && active_e && eepf, "accumulate_eepf: null pointer");
-    return launch_eepf(x, vx, vy, vz, efield, active_e, eepf, *grid, (cudaStream_t)stream);
+    return launch_eepf(EepfSamples{x, vx, vy, vz, efield, active_e, eepf, nullptr, nullptr}, *grid,
+                       (cudaStream_t)stream);
 }

@@ -17,6 +17,9 @@
 // advances the counter.
 #include "batch_internal.h"
 #include "common.cuh"
+#include <algorithm>
+
+#include "eepf.cuh"
 #include "internal.h"
 #include "poisson.cuh"
 
@@ -69,6 +72,7 @@ struct MeasureGrid {
                     for (int q = 0; q < 4; ++q) old_xt[q] = m.xt[(XT_POT + q) * plane + at];
             }
             const float v[4] = {__ldcg(pot + k), __ldcg(efield + k), __ldcg(e_density + k), __ldcg(i_density + k)};
+            if (m.ef_keep) m.ef_keep[k] = v[1];
             m.cumul_e[k] = old_e + (double)v[2];
             if (m.cumul_i) m.cumul_i[k] = old_i + (double)v[3];
             if (m.xt)
@@ -86,6 +90,29 @@ __global__ void __launch_bounds__(POIS_MAX_THREADS)
                    const float *__restrict__ pot0_table, uint32_t *__restrict__ step_counter,
                    const cudapic_grid g, float *__restrict__ zero_a, float *__restrict__ zero_b,
                    const PoissonMeasure meas) {
+    grid_dep_wait();
+    MeasureGrid mg;
+    mg.fetch(meas, step_counter, g);
+    poisson_solve<T, PT>(e_density, i_density, pot_out, efield_out, pot0_arg, pot0_table, step_counter, g, zero_a,
+                        zero_b);
+    mg.add(meas, e_density, i_density, pot_out, efield_out, g);
+}
+
+// A measured step's solve (CTA 0) beside the previous step's EEPF samples (the
+// other CTAs), which need that step's field only: in a launch of their own
+// before the solve they cost 5 us of a measured step of 400 000 particles
+// (one such cycle of 4000 steps 167 ms, now 160).
+template <typename T, int PT>
+__global__ void __launch_bounds__(POIS_MAX_THREADS)
+    poisson_eepf_kernel(const float *__restrict__ e_density, const float *__restrict__ i_density,
+                        float *__restrict__ pot_out, float *__restrict__ efield_out, float pot0_arg,
+                        const float *__restrict__ pot0_table, uint32_t *__restrict__ step_counter,
+                        const cudapic_grid g, float *__restrict__ zero_a, float *__restrict__ zero_b,
+                        const PoissonMeasure meas, const EepfSamples eepf, int vec) {
+    if (blockIdx.x > 0) {
+        eepf_accumulate(eepf, g, vec != 0, blockIdx.x - 1, gridDim.x - 1);
+        return;
+    }
     grid_dep_wait();
     MeasureGrid mg;
     mg.fetch(meas, step_counter, g);
@@ -169,26 +196,35 @@ void poisson_shape(uint32_t n_g, int &threads, int &per_thread) {
 template <typename T, int PT>
 int launch_poisson_t(const float *e_density, const float *i_density, float *pot, float *efield, float pot0,
                      const float *pot0_table, uint32_t *step_counter, const cudapic_grid &g, int threads,
-                     cudaStream_t stream, float *zero_a, float *zero_b, const PoissonMeasure &meas) {
+                     cudaStream_t stream, float *zero_a, float *zero_b, const PoissonMeasure &meas, const EepfSamples *eepf) {
     const size_t smem = poisson_solve_smem<T>(g.n_g);
-    auto kern = poisson_kernel<T, PT>;
+    if (!eepf) {
+        auto kern = poisson_kernel<T, PT>;
+        CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "poisson"));
+        return launch_kernel("solve_poisson_scan", kern, dim3(1), dim3(threads), smem, stream, e_density, i_density,
+                             pot, efield, pot0, pot0_table, step_counter, g, zero_a, zero_b, meas);
+    }
+    auto kern = poisson_eepf_kernel<T, PT>;
     CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "poisson"));
-    return launch_kernel("solve_poisson_scan", kern, dim3(1), dim3(threads), smem, stream, e_density, i_density, pot,
-                         efield, pot0, pot0_table, step_counter, g, zero_a, zero_b, meas);
+    threads = std::max(threads, 512);  // for the samples; further threads add zeros to the solve's sums
+    const uint64_t want = ((uint64_t)g.capacity + 4 * threads - 1) / (4 * threads);
+    return launch_kernel("solve_poisson_eepf", kern, dim3(1 + (unsigned)std::min<uint64_t>(2ull * sm_count() - 1, want)),
+                         dim3(threads), smem, stream, e_density, i_density, pot, efield, pot0, pot0_table,
+                         step_counter, g, zero_a, zero_b, meas, *eepf, (int)aligned16(eepf->x));
 }
 
 template <typename T>
 int launch_poisson_pt(const float *e_density, const float *i_density, float *pot, float *efield, float pot0,
                       const float *pot0_table, uint32_t *step_counter, const cudapic_grid &g,
-                      cudaStream_t stream, float *zero_a, float *zero_b, const PoissonMeasure &meas) {
+                      cudaStream_t stream, float *zero_a, float *zero_b, const PoissonMeasure &meas, const EepfSamples *eepf) {
     int threads, pt;
     poisson_shape(g.n_g, threads, pt);
     switch (pt) {
-    case 1: return launch_poisson_t<T, 1>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas);
-    case 2: return launch_poisson_t<T, 2>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas);
-    case 4: return launch_poisson_t<T, 4>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas);
-    case 8: return launch_poisson_t<T, 8>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas);
-    default: return launch_poisson_t<T, 16>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas);
+    case 1: return launch_poisson_t<T, 1>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas, eepf);
+    case 2: return launch_poisson_t<T, 2>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas, eepf);
+    case 4: return launch_poisson_t<T, 4>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas, eepf);
+    case 8: return launch_poisson_t<T, 8>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas, eepf);
+    default: return launch_poisson_t<T, 16>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, threads, stream, zero_a, zero_b, meas, eepf);
     }
 }
 
@@ -423,12 +459,13 @@ int launch_poisson_f64(const double *dens_e, const double *dens_i, double *pot, 
 
 int launch_poisson(const float *e_density, const float *i_density, float *pot, float *efield, float pot0,
                    const float *pot0_table, uint32_t *step_counter, const cudapic_grid &g,
-                   cudaStream_t stream, float *zero_a, float *zero_b, const PoissonMeasure &meas) {
+                   cudaStream_t stream, float *zero_a, float *zero_b, const PoissonMeasure &meas,
+                   const EepfSamples *eepf) {
     if (g.n_g > (uint32_t)(POIS_MAX_THREADS * POIS_MAX_PER_THREAD))
         return fail(CUDAPIC_ERR_ARG, "solve_poisson: n_g > 16384");
     if (g.flags & CUDAPIC_FLAG_POISSON_F32_SCAN)
-        return launch_poisson_pt<float>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, stream, zero_a, zero_b, meas);
-    return launch_poisson_pt<double>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, stream, zero_a, zero_b, meas);
+        return launch_poisson_pt<float>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, stream, zero_a, zero_b, meas, eepf);
+    return launch_poisson_pt<double>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, stream, zero_a, zero_b, meas, eepf);
 }
 
 // Batched solve: CTA d solves discharge d of the batch (the driver variant
@@ -451,7 +488,8 @@ __global__ void __launch_bounds__(POIS_MAX_THREADS)
     }
     const float *e_dens = dd.e_dens[e_read];
     const float *i_dens = dd.i_dens[i_read];
-    const PoissonMeasure meas = measure ? PoissonMeasure{dd.cumul_e, ion_step ? dd.cumul_i : nullptr, dd.xt, dd.n_xt}
+    const PoissonMeasure meas = measure ? PoissonMeasure{dd.cumul_e, ion_step ? dd.cumul_i : nullptr, dd.xt, dd.n_xt,
+                                                       nullptr}
                                         : PoissonMeasure{};
     MeasureGrid mg;
     mg.fetch(meas, ctr + 3, s_g);

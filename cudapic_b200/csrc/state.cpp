@@ -106,6 +106,13 @@ void destroy_graphs(cudapic_state *s) {
     }
 }
 
+// The EEPF samples of the electrons as they are, with the field that pushed them.
+EepfSamples eepf_samples(const cudapic_state *s, const float *efield) {
+    const int se = s->side[0];
+    return EepfSamples{s->x[0][se], s->vx[0][se], s->vy[0][se], s->vz[0][se], efield, s->n_e(), s->eepf, s->esum,
+                       s->mcount + 2};
+}
+
 // Particle part of a fused-mode step: [ion push] -> electron step ->
 // [ion collisions] -> [measurement]; the kernels publish the particle counts
 // themselves (StepLink), so the step holds no copy or memset node.  The
@@ -202,9 +209,11 @@ int enqueue_fused_particles(cudapic_state *s, bool ion_step, float *e_next, floa
                                           s->vz[I][si], s->rng[I][0], s->rng[I][1], s->rng[I][2], s->rng[I][3],
                                           nullptr, g, st, s->measure ? s->mcount + 1 : nullptr, s->ion_k));
     }
+    // the EEPF samples: beside the next step's solve when that is enqueued next
+    // (a compacting step may be the last one before a graph)
     if (s->measure) {
-        CUDAPIC_CHECK(launch_eepf(s->x[E][se], s->vx[E][se], s->vy[E][se], s->vz[E][se], s->efield, s->n_e(),
-                                  s->eepf, g, st, s->esum, s->mcount + 2));
+        if (next_ion >= 0 && !compact) s->eepf_pending = true;
+        else CUDAPIC_CHECK(launch_eepf(eepf_samples(s, s->efield), g, st));
     }
     return CUDAPIC_OK;
 }
@@ -247,12 +256,19 @@ int enqueue_step(cudapic_state *s, bool ion_step, bool compact, int next_ion) {
         }
         i_acc = s->i_dens[s->i_cur ^ 1];
     }
-    if (!s->poisson_ahead)  // else the previous step's scatter pass solved it, and cleared the collectors
+    if (!s->poisson_ahead) {  // else the previous step's scatter pass solved it, and cleared the collectors
+        // the previous step's EEPF samples still to be taken: with that step's
+        // field, which its solve kept beside the one overwritten here
+        const bool samples = s->eepf_pending;
+        s->eepf_pending = false;
+        const EepfSamples eepf = eepf_samples(s, s->ef_keep[s->e_cur ^ 1]);
         CUDAPIC_CHECK(launch_poisson(s->e_density(), s->i_density(), s->pot, s->efield, 0.0f, s->pot0_table,
                                      s->step_counter(), g, st, e_next, zero_b,
                                      s->measure ? PoissonMeasure{s->cumul_e, ion_step ? s->cumul_i : nullptr, s->xt,
-                                                                 s->n_xt}
-                                                : PoissonMeasure{}));
+                                                                 s->n_xt, s->ef_keep[s->e_cur]}
+                                                : PoissonMeasure{},
+                                     samples ? &eepf : nullptr));
+    }
     s->poisson_ahead = false;
     if (s->measure) {
         if (s->xt) {  // XT diagnostics: the particles before their push
@@ -303,10 +319,7 @@ int enqueue_step(cudapic_state *s, bool ion_step, bool compact, int next_ion) {
                                           s->vz[I][si], s->rng[I][0], s->rng[I][1], s->rng[I][2], s->rng[I][3],
                                           nullptr, g, st, s->measure ? s->mcount + 1 : nullptr));
     }
-    if (s->measure) {
-        CUDAPIC_CHECK(launch_eepf(s->x[E][se], s->vx[E][se], s->vy[E][se], s->vz[E][se], s->efield, s->n_e(),
-                                  s->eepf, g, st, s->esum, s->mcount + 2));
-    }
+    if (s->measure) CUDAPIC_CHECK(launch_eepf(eepf_samples(s, s->efield), g, st));
     return CUDAPIC_OK;
 }
 
@@ -337,6 +350,7 @@ int build_graph(cudapic_state *s) {
     cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
     // a graph of 2 N_SUB steps returns every ping-pong role to its start
     s->poisson_ahead = false;  // the last captured step solved nothing ahead (a failed capture may have)
+    s->eepf_pending = false;
     s->side[0] = side0[0];
     s->side[1] = side0[1];
     s->e_cur = cur0[0];
@@ -461,7 +475,8 @@ extern "C" int cudapic_state_create(const cudapic_params *p, int device, cudapic
             if ((rc = dalloc(s, &s->rng[sp][k], cap))) return cleanup(rc);
     }
     const size_t n_g = p->n_g;
-    if ((rc = dalloc(s, &s->counters, 64)) || (rc = dalloc(s, &s->efield, n_g)) || (rc = dalloc(s, &s->pot, n_g)) ||
+    if ((rc = dalloc(s, &s->counters, 64)) || (rc = dalloc(s, &s->efield, n_g)) ||
+        (rc = dalloc(s, &s->ef_keep[0], n_g)) || (rc = dalloc(s, &s->ef_keep[1], n_g)) || (rc = dalloc(s, &s->pot, n_g)) ||
         (rc = dalloc(s, &s->e_dens[0], n_g)) || (rc = dalloc(s, &s->e_dens[1], n_g)) ||
         (rc = dalloc(s, &s->i_dens[0], n_g)) || (rc = dalloc(s, &s->i_dens[1], n_g)) ||
         (rc = dalloc(s, &s->pot0_table, p->n_t)) || (rc = dalloc(s, &s->cs, 5ull * CUDAPIC_CS_RANGES)) ||

@@ -38,6 +38,11 @@ struct cudapic_state {
     // solve already enqueued by the step before it
     bool solve_ahead = true;
     bool poisson_ahead = false;
+    // measurement: the field of the step whose densities are e_dens[e_cur], kept
+    // for its EEPF samples; eepf_pending: the step being enqueued takes the
+    // previous step's samples beside its solve
+    float *ef_keep[2] = {};
+    bool eepf_pending = false;
     bool dens_valid = false;  // e_dens[e_cur] and both ion buffers describe the particles
     int graph_key[2][4] = {{-1, -1, -1, -1}, {-1, -1, -1, -1}};  // sides and buffer roles at capture
     float *cs = nullptr, *sigma_tot_e = nullptr, *sigma_tot_i = nullptr;

@@ -325,6 +325,36 @@ def test_measurement_accumulators(cudapic, cuda_device):
     st.close()
 
 
+@pytest.mark.parametrize("n,n_g", [(3, 5), (2047, 511), (40_003, 400), (40_003, 513), (100_001, 1100)])
+def test_eepf_beside_the_next_solve_equals_a_launch_of_its_own(cudapic, cuda_device, n, n_g):
+    """65 measured steps in one call (samples taken beside the next step's
+    solve, in a graph and out of one) and in 65 (each in a launch of its own):
+    in the vacuum field of 250 V, which changes every step, without gas or
+    charge, both push the same electrons bit for bit, so the histograms are
+    equal and the energy sums up to the order of their additions."""
+    from cudapic_b200.sim import GpuSimState, ParticlesSoA
+    params = cudapic.default_params(capacity=40_000 if n < 32_000 else (n + 11) // 4 * 4, n_g=n_g, pressure=1e-9, weight=1e-20)
+    rng = np.random.default_rng(n)
+    x = (0.025 * rng.uniform(0.3, 0.7, n)).astype(np.float32)
+    x[:3] = 0.0125
+    v = rng.normal(0.0, 5e5, (3, n)).astype(np.float32)
+    out = []
+    for calls in (1, 65):
+        st = GpuSimState(params)
+        st.upload_electrons(ParticlesSoA(x, *v))
+        st.upload_ions(ParticlesSoA(x[:1], *(np.zeros(1, np.float32) for _ in range(3))))
+        st.seed()
+        st.set_measure(True)
+        for _ in range(calls):
+            st.run_steps(65 // calls)
+        assert st.counts() == (n, 1) and st.device_error() == 0
+        _, _, eepf = st.download_measurements()
+        out.append((eepf, st.report()["mean_energy_center"]))
+        st.close()
+    assert out[0][0].sum() >= 65 and np.array_equal(out[0][0], out[1][0])
+    assert out[0][1] == pytest.approx(out[1][1], rel=1e-12)
+
+
 def test_c1_population_steps_without_device_errors(cudapic, cuda_device):
     from cudapic_b200.sim import GpuSimState, ParticlesSoA
     from cudapic_b200.workloads import steady_state
