@@ -226,18 +226,6 @@ constexpr int MS_CLUSTER = 2;                   // the largest that still reache
 constexpr uint32_t MS_TABLE = 32768;            // entries whose maximum a launch looks for
 constexpr float MS_TABLE_EV = 32.7f;            // energies below have an index below MS_TABLE
 
-// True when the ion certainly does not collide, u the test draw (the fifth):
-// ion_collides decides so for u >= k (|v| + 9.2 sigma) + 6e-7.  Without the
-// root: with c >= 9.2 sigma k + 6.5e-7 and k2 >= k^2 (1 + 1e-4), y = fl(u - c)
-// >= 0 and fl(y y) >= fl(k2 v2) give y >= k |v| (each rounding is within
-// 2^-24 relative), hence u >= k |v| + c - 2^-24 > k (|v| + 9.2 sigma) + 5.8e-7,
-// which exceeds the computed collision probability (at most k (|v| + 9.2
-// sigma) + 3.1e-7).  NaN or infinite constants decide nothing.
-__device__ __forceinline__ bool ion_surely_passes(float u, float v2, float k2, float c) {
-    const float y = u - c;
-    return y >= 0.0f && y * y >= k2 * v2;
-}
-
 template <bool ION, bool EVENTS, bool BOUNDED>
 __global__ void __launch_bounds__(MS_THREADS, 1)
     check_collisions_stream_kernel(const float *__restrict__ sigma_tot, const float *__restrict__ cs,
@@ -296,8 +284,8 @@ __global__ void __launch_bounds__(MS_THREADS, 1)
             v2_max = MS_TABLE_EV / g.half_me_over_e;
         }
     }
-    const float k2 = k * k * 1.0001f;                                       // the bound on (nu dt)^2 / v.v
-    const float c = fmaf(k, 9.2f * g.normal_range, 6.5e-7f) * 1.000001f;    // ions: beside it
+    const float k2 = k * k * 1.0001f;                 // the bound on (nu dt)^2 / v.v
+    const float c = ion_bound_offset(k, g.normal_range);  // ions: beside it
     const GlobalTable table{sigma_tot};
     // the four particles of a lane: neighbours for the vector loads, else 32
     // apart, so that the scalar loads of a warp meet

@@ -350,6 +350,21 @@ __device__ __forceinline__ bool ion_collides(float vxi, float vyi, float vzi, Xo
     return test_ion(vxi, vyi, vzi, rs, sigma_tot_i, g).collide;
 }
 
+// True when the ion certainly does not collide, u the test draw (the fifth):
+// ion_collides decides so for u >= k (|v| + 9.2 sigma) + 6e-7.  Without the
+// root: with c >= 9.2 sigma k + 6.5e-7 and k2 >= k^2 (1 + 1e-4), y = fl(u - c)
+// >= 0 and fl(y y) >= fl(k2 v2) give y >= k |v| (each rounding is within
+// 2^-24 relative), hence u >= k |v| + c - 2^-24 > k (|v| + 9.2 sigma) + 5.8e-7,
+// which exceeds the computed collision probability (at most k (|v| + 9.2
+// sigma) + 3.1e-7).  NaN or infinite constants decide nothing.
+__device__ __forceinline__ bool ion_surely_passes(float u, float v2, float k2, float c) {
+    const float y = u - c;
+    return y >= 0.0f && y * y >= k2 * v2;
+}
+__device__ __forceinline__ float ion_bound_offset(float k, float normal_range) {
+    return fmaf(k, 9.2f * normal_range, 6.5e-7f) * 1.000001f;
+}
+
 // collision_i, Rust-CUDA/src/main.rs:1221-1292; returns 4 isotropic, 5 backscatter.
 static __device__ __noinline__ uint32_t collide_ion(uint32_t i, uint32_t idx, float vxi, float vyi, float vzi, float vxa,
                                              float vya, float vza, Xoshiro128p &rs, const float *__restrict__ cs,

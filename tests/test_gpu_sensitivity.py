@@ -67,7 +67,7 @@ def test_forward_bit_exact_against_oracle(cudapic, cuda_device, oracle, tables):
 @pytest.mark.parametrize("n", [1, 255, 1025, 2_500_000])
 def test_forward_sizes_bit_exact(cudapic, cuda_device, oracle, tables, n):
     """One ion cycle from a single particle to more rounds per CTA (17 of
-    256 slots) than a 32-bit deposit histogram takes without a drain (15).
+    1024 slots) than a 32-bit deposit histogram takes without a drain (3).
     RNG states bit for bit.  Positions: the FP64 field sums run in another
     order than the oracle's, so a node's f32 field may round the other way:
     one ulp of at most 1e6 V/m in each of 20 steps moves a particle by at
