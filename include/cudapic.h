@@ -485,7 +485,12 @@ int cudapic_state_seed(cudapic_state *s, const uint32_t e_master[4], const uint3
  * (accumulate_density + accumulate_eepf, Rust-CUDA/src/main.rs:1746-1756, 1802-1807). */
 int cudapic_state_set_measure(cudapic_state *s, int on);
 /* Enqueues n_steps reference-order time steps (Rust-CUDA/src/main.rs:1728-1807)
- * on the state's stream.  Asynchronous. */
+ * on the state's stream.  Asynchronous.  With every switch below at its default,
+ * not measuring, a capacity of at most 32 688 and N_G <= 1024, whole ion cycles
+ * (N_SUB steps from a multiple of N_SUB on) run in one launch of one
+ * thread-block cluster, with the same steps and the electrons compact at the
+ * end of every cycle; the rest of a run, and every other state, in the
+ * launches described below. */
 int cudapic_state_run_steps(cudapic_state *s, uint64_t n_steps);
 /* on (default): each step runs the fused electron kernel
  * (cudapic_step_electrons: push, collisions and the next step's deposit in
