@@ -23,10 +23,12 @@
 // shared f32 atomics (eight per electron; the two of the ionization rate only
 // above the threshold, below which the table is zero) and by latency: with
 // 512 threads and one particle per thread and round, every round waiting for
-// its loads, 400 000 electrons took 15.9 us, now 11.3 us.
+// its loads, 400 000 electrons took 15.9 us, now 11.3 us (alone).
 // The grid quantities are added by the solve's launch (kernels_poisson.cu).
 // The batched variant walks each CTA's share of the batch's concatenated
 // particles discharge by discharge (one flush per segment).
+#include <algorithm>
+
 #include "batch_internal.h"
 #include "common.cuh"
 #include "internal.h"
@@ -190,8 +192,14 @@ __global__ void __launch_bounds__(XT_THREADS)
 int launch_xt_particles(bool ions, const float *x, const float *vx, const float *vy, const float *vz,
                         const uint32_t *n_active, const float *efield, const float *cs, const uint32_t *step_counter,
                         const cudapic_grid &g, uint32_t n_xt, double *xt, cudaStream_t stream) {
-    const size_t smem = (size_t)(ions ? 3 : 4) * g.n_g * sizeof(float);
-    if (smem > (size_t)max_smem_optin()) return fail(CUDAPIC_ERR_ARG, "xt: n_g too large");
+    const size_t need = (size_t)(ions ? 3 : 4) * g.n_g * sizeof(float);
+    if (need > (size_t)max_smem_optin()) return fail(CUDAPIC_ERR_ARG, "xt: n_g too large");
+    // at least half of an SM's shared memory, so that no SM takes two CTAs:
+    // under programmatic dependent launch the CTAs are placed while the
+    // solve's launch still holds some SMs, two fit by registers, and the SMs
+    // with two then set the pace (a measured step of 2 M electrons took 123 us
+    // in the driver, now 90; 400 000: 41.9, now 35.5)
+    const size_t smem = std::max(need, (size_t)max_smem_optin() / 2 + 1024);
     auto kern = ions ? xt_particles_kernel<true> : xt_particles_kernel<false>;
     CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "xt"));
     const unsigned grid = persistent_grid(1, ((uint64_t)g.capacity + XT_THREADS - 1) / XT_THREADS);
