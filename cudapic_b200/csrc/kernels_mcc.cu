@@ -226,6 +226,13 @@ constexpr int MS_CLUSTER = 2;                   // the largest that still reache
 constexpr uint32_t MS_TABLE = 32768;            // entries whose maximum a launch looks for
 constexpr float MS_TABLE_EV = 32.7f;            // energies below have an index below MS_TABLE
 
+// The larger of two floats, NaN (the canonical one, 0x7fffffff) if either is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+
 template <bool ION, bool EVENTS, bool BOUNDED>
 __global__ void __launch_bounds__(MS_THREADS, 1)
     check_collisions_stream_kernel(const float *__restrict__ sigma_tot, const float *__restrict__ cs,
@@ -260,11 +267,12 @@ __global__ void __launch_bounds__(MS_THREADS, 1)
         cg::cluster_group cluster = cg::this_cluster();
         constexpr uint32_t part = MS_TABLE / MS_CLUSTER;
         const float *mine = sigma_tot + cluster.block_rank() * part;
-        // entries compared as bit patterns: for non-negative floats their
-        // order; a negative or NaN entry makes a bound that decides nothing
-        uint32_t top = 0;
+        // the largest of +0 and the entries: an entry below zero (or -0) never
+        // lets a particle collide, a NaN stays and makes a bound that decides nothing
+        float largest = 0.0f;
 #pragma unroll
-        for (uint32_t q = 0; q < part / MS_THREADS; ++q) top = max(top, __float_as_uint(__ldg(mine + q * MS_THREADS + tid)));
+        for (uint32_t q = 0; q < part / MS_THREADS; ++q) largest = max_nan(largest, __ldg(mine + q * MS_THREADS + tid));
+        uint32_t top = __float_as_uint(largest);  // non-negative or the canonical NaN: ordered as integers
         top = __reduce_max_sync(0xffffffffu, top);
         if (lane == 0) s_max[warp] = top;
         __syncthreads();

@@ -701,6 +701,38 @@ def test_check_collisions_tile_edges(cudapic, K, oracle, dev_tables, tables, spe
         assert np.array_equal(_read(d)[:n].view(np.uint32), h[:n].view(np.uint32))
 
 
+@pytest.mark.parametrize("species", ["e", "i"])
+@pytest.mark.parametrize("entry", [-0.0, -1e-30, -5e4, np.nan, -np.nan, np.inf])
+def test_check_collisions_odd_table_entry(cudapic, K, oracle, dev_tables, tables, species, entry):
+    """One entry of the caller's table that no cross section gives (a zero
+    with its sign set, a negative number, NaN, infinity) where the launch
+    looks for the largest: every other particle's test is as before."""
+    cs, se, si = tables
+    dcs, _, _ = dev_tables
+    n = 20_011
+    g = cudapic.grid_from_params(n_t=200, capacity=n)
+    ph = oracle.phys_from_params(n_t=200, capacity=n)
+    x, vx, vy, vz = _mcc_case(n, 5.0 if species == "e" else 0.5, n, E_MASS if species == "e" else AR_MASS)
+    tab = (se if species == "e" else si).copy()
+    tab[1000] = entry
+    r_h = [np.asarray(p).copy() for p in oracle.seed_streams([4, 3, 2, 1], n)]
+    v_h = [vx.copy(), vy.copy(), vz.copy()]
+    planes = [dev(a) for a in v_h + r_h]
+    events = zeros(n, np.uint8)
+    if species == "e":
+        e_h, i_h = [x.copy()] + v_h, [np.zeros(n, np.float32) for _ in range(4)]
+        K.check_collisions_e(dev(tab), dcs, counter(n), dev(x), *planes, *[zeros(n) for _ in range(4)], counter(n),
+                             counter(0), g, events=events)
+        ev_ref, _, _, _ = oracle.check_collisions_e(tab, cs, n, e_h, r_h, i_h, n, 0, ph)
+    else:
+        K.check_collisions_i(dev(tab), dcs, counter(n), *planes, g, events=events)
+        ev_ref = oracle.check_collisions_i(tab, cs, n, v_h, r_h, ph)
+    assert (ev_ref > 0).sum() > 100
+    assert np.array_equal(host(events), ev_ref)
+    for d, h in zip(planes, v_h + r_h):
+        assert np.array_equal(host(d).view(np.uint32), h.view(np.uint32))
+
+
 def test_spawn_capacity_is_enforced(cudapic, K, oracle, dev_tables, tables):
     """Ionization spawns beyond capacity are dropped and flagged, never
     written past the buffers (the reference writes unbounded)."""
