@@ -345,6 +345,9 @@ __global__ void __launch_bounds__(IP_THREADS)
 // atom for every ion and scalar loads 104 us, now 85.
 constexpr uint32_t BC_TILE = 128;           // slots per warp and round
 constexpr int BC_QCAP = 32 + (int)BC_TILE;  // a warp drains at 32; one tile adds <= 128
+// undecided ions of a tile beyond which they are tested in place (kernels_mcc.cu
+// MS_DENSE_I): 24 discharges at 1500 Pa 278 us by the queues alone, now 183
+constexpr int BC_DENSE = 48;
 
 struct IonCollIO {
     float *vx, *vy, *vz;
@@ -460,6 +463,7 @@ __global__ void __launch_bounds__(ES_THREADS)
                     open |= 1u << u;
                 }
             }
+            if (__reduce_add_sync(0xffffffffu, __popc(open)) > BC_DENSE) settle_ions(open, v, s, table, g);
             if (any) {
                 *reinterpret_cast<uint4 *>(io.rng0 + i0) = make_uint4(s[0][0], s[0][1], s[0][2], s[0][3]);
                 *reinterpret_cast<uint4 *>(io.rng1 + i0) = make_uint4(s[1][0], s[1][1], s[1][2], s[1][3]);

@@ -208,7 +208,8 @@ __global__ void __launch_bounds__(MCC_THREADS, 4)
 //  * undecided particles go to a queue private to their warp (slot and RNG
 //    state before the test); whenever it holds 32 the warp takes 32 of them,
 //    one per lane, through the full test and, colliding, the scattering --
-//    only __syncwarp, no block-wide synchronisation.
+//    only __syncwarp, no block-wide synchronisation.  A tile with many of them
+//    takes the full test first and queues its colliders (MS_DENSE_E).
 // Bound by memory (44 B per particle).  With the first 32768 entries copied to
 // every SM's shared memory and the full test on every particle (128 KB per
 // CTA and launch, scalar loads, a square root and a division each) 2 000 001
@@ -225,6 +226,14 @@ constexpr size_t MS_SMEM = (size_t)MS_WARPS * 5 * MS_QCAP * sizeof(uint32_t);
 constexpr int MS_CLUSTER = 2;                   // the largest that still reaches every SM (4 leaves some idle)
 constexpr uint32_t MS_TABLE = 32768;            // entries whose maximum a launch looks for
 constexpr float MS_TABLE_EV = 32.7f;            // energies below have an index below MS_TABLE
+// Undecided particles of a tile beyond which all of its undecided take the
+// full test where they are: a queue's particles are gathered again, 32 at a
+// time, which pays for a few of 128 and not for a hot or strongly collisional
+// population.  2 000 001 electrons of 3 / 30 / 1000 eV (a call, 10 Pa) took 31 /
+// 82 / 118 us by the queue alone, now 31 / 43 / 42 (37 / 45 / 47 with the full
+// test on every particle); ions of 500 eV at 100 Pa, bounded, 77, now 54 (63).
+// Between the two forms the calls cross at a quarter to a half of a tile.
+constexpr int MS_DENSE_E = 32, MS_DENSE_I = 48;
 
 // The larger of two floats, NaN (the canonical one, 0x7fffffff) if either is.
 __device__ __forceinline__ float max_nan(float a, float b) {
@@ -332,6 +341,9 @@ __global__ void __launch_bounds__(MS_THREADS, 1)
     };
 
     uint32_t qn = 0;  // entries in this warp's queue (warp-uniform)
+    // ions: this warp met a tile beyond MS_DENSE_I; its further tiles skip the bound (50 eV at 100 Pa, unbounded,
+    // 54 us with it, 51 without; for electrons the flag cost 2 to 8 %)
+    bool dense = false;
     // tile t to CTA t mod gridDim: every SM gets the same number to within one
     const uint32_t tiles = (uint32_t)(((uint64_t)n + MS_TILE - 1) / MS_TILE);
     for (uint32_t t = blockIdx.x + (uint32_t)warp * gridDim.x; t < tiles; t += gridDim.x * MS_WARPS) {
@@ -364,29 +376,41 @@ __global__ void __launch_bounds__(MS_THREADS, 1)
                 s[3][u] = in ? rng3[i0 + u * di] : 0u;
             }
         }
-        uint32_t open = 0;  // bit u: not decided by the bound (its state stays before the test)
+        uint32_t open = 0xfu;  // bit u: not decided by the bound (its state stays before the test)
+        if (!whole) {
 #pragma unroll
-        for (int u = 0; u < MS_ROW; ++u) {
-            const float v2 = v[0][u] * v[0][u] + v[1][u] * v[1][u] + v[2][u] * v[2][u];
-            Xoshiro128p rs{s[0][u], s[1][u], s[2][u], s[3][u]};
-            bool passes;
-            if (ION) {
-                rs.next();  // the target atom's four draws
-                rs.next();
-                rs.next();
-                rs.next();
-                passes = ion_surely_passes(rs.uniform(), v2, k2, c);
-            } else {
-                passes = !may_collide(rs.uniform(), v2, k2);
+            for (uint32_t u = 0; u < MS_ROW; ++u)
+                if (i0 + u * di >= n) open &= ~(1u << u);
+        }
+        if (!dense) {
+#pragma unroll
+            for (int u = 0; u < MS_ROW; ++u) {
+                const float v2 = v[0][u] * v[0][u] + v[1][u] * v[1][u] + v[2][u] * v[2][u];
+                Xoshiro128p rs{s[0][u], s[1][u], s[2][u], s[3][u]};
+                bool passes;
+                if (ION) {
+                    rs.next();  // the target atom's four draws
+                    rs.next();
+                    rs.next();
+                    rs.next();
+                    passes = ion_surely_passes(rs.uniform(), v2, k2, c);
+                } else {
+                    passes = !may_collide(rs.uniform(), v2, k2);
+                }
+                if (passes && (BOUNDED || v2 < v2_max)) {
+                    s[0][u] = rs.s0;
+                    s[1][u] = rs.s1;
+                    s[2][u] = rs.s2;
+                    s[3][u] = rs.s3;
+                    open &= ~(1u << u);
+                }
             }
-            if (passes && (BOUNDED || v2 < v2_max)) {
-                s[0][u] = rs.s0;
-                s[1][u] = rs.s1;
-                s[2][u] = rs.s2;
-                s[3][u] = rs.s3;
-            } else if (i0 + (uint32_t)u * di < n) {
-                open |= 1u << u;
-            }
+        }
+        if (ION) {
+            dense = dense || __reduce_add_sync(0xffffffffu, __popc(open)) > MS_DENSE_I;
+            if (dense) settle_ions(open, v, s, table, g);
+        } else if (__reduce_add_sync(0xffffffffu, __popc(open)) > MS_DENSE_E) {
+            settle_electrons(open, v, s, table, g);
         }
         if (whole) {  // open ones keep their state until their drain
             *reinterpret_cast<uint4 *>(rng0 + i0) = make_uint4(s[0][0], s[0][1], s[0][2], s[0][3]);
@@ -419,14 +443,6 @@ __global__ void __launch_bounds__(MS_THREADS, 1)
                     wq[2 * MS_QCAP + q] = s[1][u];
                     wq[3 * MS_QCAP + q] = s[2][u];
                     wq[4 * MS_QCAP + q] = s[3][u];
-                    if (!ION) {  // the drain's gathers, fetched together instead of one after the other
-                        const float v2 = v[0][u] * v[0][u] + v[1][u] * v[1][u] + v[2][u] * v[2][u];
-                        const uint32_t e = energy_index(g.half_me_over_e * v2);
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(sigma_tot + e));
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(cs + e));
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(cs + CS_RANGES + e));
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(cs + 2 * CS_RANGES + e));
-                    }
                 }
                 qn += __popc(m);
             }

@@ -365,6 +365,53 @@ __device__ __forceinline__ float ion_bound_offset(float k, float normal_range) {
     return fmaf(k, 9.2f * normal_range, 6.5e-7f) * 1.000001f;
 }
 
+// The full test of a lane's particles that the certain rejection left open
+// (bit u of `open`; states s[.][u] before the test): those that do not collide
+// get their advanced state and leave `open`.  Electrons two at a time: their
+// lookups together; four at a time spilled registers (3 us of 46).
+template <typename Table>
+__device__ __forceinline__ void settle_electrons(uint32_t &open, const float (&v)[3][4], uint32_t (&s)[4][4],
+                                                 const Table &sigma_tot_e, const cudapic_grid &g) {
+#pragma unroll
+    for (int h = 0; h < 4; h += 2) {
+        float v2[2], sigma[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int u = h + q;
+            v2[q] = v[0][u] * v[0][u] + v[1][u] * v[1][u] + v[2][u] * v[2][u];
+            sigma[q] = sigma_tot_e(energy_index(g.half_me_over_e * v2[q]));
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int u = h + q;
+            if (!(open >> u & 1u)) continue;
+            Xoshiro128p rs{s[0][u], s[1][u], s[2][u], s[3][u]};
+            const float nu = sigma[q] * sqrtf(v2[q]);
+            if (collision_draw(rs.uniform(), nu * g.dt_e)) continue;
+            s[0][u] = rs.s0;
+            s[1][u] = rs.s1;
+            s[2][u] = rs.s2;
+            s[3][u] = rs.s3;
+            open &= ~(1u << u);
+        }
+    }
+}
+template <typename Table>
+__device__ __forceinline__ void settle_ions(uint32_t &open, const float (&v)[3][4], uint32_t (&s)[4][4],
+                                            const Table &sigma_tot_i, const cudapic_grid &g) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        if (!(open >> u & 1u)) continue;
+        Xoshiro128p rs{s[0][u], s[1][u], s[2][u], s[3][u]};
+        if (test_ion(v[0][u], v[1][u], v[2][u], rs, sigma_tot_i, g).collide) continue;
+        s[0][u] = rs.s0;
+        s[1][u] = rs.s1;
+        s[2][u] = rs.s2;
+        s[3][u] = rs.s3;
+        open &= ~(1u << u);
+    }
+}
+
 // collision_i, Rust-CUDA/src/main.rs:1221-1292; returns 4 isotropic, 5 backscatter.
 static __device__ __noinline__ uint32_t collide_ion(uint32_t i, uint32_t idx, float vxi, float vyi, float vzi, float vxa,
                                              float vya, float vza, Xoshiro128p &rs, const float *__restrict__ cs,

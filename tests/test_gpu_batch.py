@@ -121,6 +121,48 @@ def test_batch_first_step_bit_exact_against_each_discharge_alone(cudapic, cuda_d
             st.close()
 
 
+def test_batch_ion_collisions_of_dense_tiles(cudapic, cuda_device, oracle):
+    """Gas so dense that the certain rejection leaves most ions of a tile
+    open (tested in place) or about a third (on either side of the rule),
+    without electrons: after one step every ion's velocity and stream as the
+    oracle's, whose ions are those of the same step without gas, in the slots
+    that the batch gave them (their positions tell them apart)."""
+    from cudapic_b200.sim import GpuBatch
+    cases = [(400, 0, 1500, 250.0, 900.0, 0.025), (200, 0, 131, 120.0, 3000.0, 0.018),
+             (800, 0, 1789, 480.0, 180.0, 0.038), (400, 0, 1021, 300.0, 140.0, 0.022)]
+    together = [_state(c, k) for k, c in enumerate(cases)]
+    alone = [_state((*c[:4], 1e-9, c[5]), k) for k, c in enumerate(cases)]
+    try:
+        rng0 = [[_plane(st.buffers().rng[1][k], st.capacity, np.uint32) for k in range(4)] for st in together]
+        with GpuBatch(together) as b:
+            b.run_steps(1)
+            b.synchronize()
+        for k, (x, y) in enumerate(zip(together, alone)):
+            y.run_steps(1)
+            got, n = x.download_ions()
+            pushed, m = y.download_ions()
+            assert n == m and x.device_error() == 0
+            at, of = np.argsort(got.x), np.argsort(pushed.x)
+            np.testing.assert_array_equal(got.x[at], pushed.x[of])
+            assert np.all(np.diff(got.x[at]) > 0)
+            v = [np.empty(n, np.float32) for _ in range(3)]
+            for d, s in zip(v, (pushed.vx, pushed.vy, pushed.vz)):
+                d[at] = s[of]
+            ph = oracle.phys_from_params(voltage=cases[k][3], pressure=cases[k][4], gap=cases[k][5], n_g=cases[k][0],
+                                         capacity=2048, weight=7.0e4)
+            cs, _, si = oracle.cross_sections(ph.gas_density)
+            rng = [p[:n].copy() for p in rng0[k]]
+            events = oracle.check_collisions_i(si, cs, n, v, rng, ph)
+            assert np.count_nonzero(events) > 0
+            for d, r in zip((got.vx, got.vy, got.vz), v):
+                np.testing.assert_array_equal(d, r, err_msg="discharge %d" % k)
+            for p, r in zip(x.buffers().rng[1], rng):
+                np.testing.assert_array_equal(_plane(p, n, np.uint32), r, err_msg="discharge %d" % k)
+    finally:
+        for st in together + alone:
+            st.close()
+
+
 def test_batch_measurements_match_each_discharge_alone(cudapic, cuda_device):
     """The measurement window of a batched step (electrode counters and
     IFEDs, collision counts, time-averaged densities, EEPF) equals the
