@@ -712,37 +712,56 @@ int resident_cluster(const cudapic_grid &g) {
     return need <= 8 * RS_FILL ? 8 : need <= 16 * RS_FILL ? 16 : 0;
 }
 
+uint32_t resident_ef_pad(const cudapic_grid &g) { return (g.n_g + 3u) & ~3u; }
+
+// A cluster's launch; the caller's `attr` outlives it.
 template <int C>
-int launch_resident_t(const ResidentArgs &a, const cudapic_grid &g, uint32_t steps, cudaStream_t stream) {
-    const uint32_t ef_pad = (g.n_g + 3u) & ~3u;
-    const size_t smem = resident_smem(ef_pad);
-    auto kern = discharge_resident_kernel<C>;
-    if (C > 8)  // beyond the portable size
-        CUDAPIC_CHECK(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
-                                 "cudaFuncSetAttribute(resident steps)"));
-    int clusters = 0;
-    CUDAPIC_CHECK(kernel_clusters((const void *)kern, RS_THREADS, smem, C, &clusters,
-                                  "cudaOccupancyMaxActiveClusters(resident steps)"));
-    if (clusters < 1) return fail(CUDAPIC_ERR_NOT_SUPPORTED, "resident steps: no resident cluster");
+cudaLaunchConfig_t resident_config(const cudapic_grid &g, cudaStream_t stream, cudaLaunchAttribute &attr) {
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = C;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(RS_THREADS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = resident_smem(resident_ef_pad(g));
     cfg.stream = stream;
-    cfg.attrs = attr;
+    cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return check_cuda(cudaLaunchKernelEx(&cfg, kern, a, g, steps, ef_pad), "launch resident steps");
+    return cfg;
+}
+
+template <int C>
+bool resident_launchable_t(const cudapic_grid &g, cudaStream_t stream) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = resident_config<C>(g, stream, attr);
+    auto kern = discharge_resident_kernel<C>;
+    int clusters = 0;
+    const bool ok = cfg.dynamicSmemBytes <= (size_t)max_smem_optin() &&
+                    kernel_smem((const void *)kern, cfg.dynamicSmemBytes, "resident steps") == CUDAPIC_OK &&
+                    // beyond the portable size of 8
+                    (C <= 8 || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+                    cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters >= 1;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
+template <int C>
+int launch_resident_t(const ResidentArgs &a, const cudapic_grid &g, uint32_t steps, cudaStream_t stream) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = resident_config<C>(g, stream, attr);
+    return check_cuda(cudaLaunchKernelEx(&cfg, discharge_resident_kernel<C>, a, g, steps, resident_ef_pad(g)),
+                      "launch resident steps");
 }
 
 }  // namespace
 
 bool resident_fits(const cudapic_grid &g, uint32_t n_sub) {
     return g.n_g <= RS_MAX_NG && n_sub >= 2 && !(g.flags & CUDAPIC_FLAG_POISSON_F32_SCAN) && resident_cluster(g) != 0;
+}
+
+bool resident_launchable(const cudapic_grid &g, cudaStream_t stream) {
+    return resident_cluster(g) == 8 ? resident_launchable_t<8>(g, stream) : resident_launchable_t<16>(g, stream);
 }
 
 int launch_resident(const ResidentArgs &a, const cudapic_grid &g, uint32_t steps, cudaStream_t stream) {

@@ -34,8 +34,12 @@ struct ResidentArgs {
 // planes assumed): capacity and grid fit the cluster's shared memory, FP64
 // Poisson sums, at least two steps per ion cycle.
 bool resident_fits(const cudapic_grid &g, uint32_t n_sub);
+// True when its cluster can be resident where `stream` launches: a stream or a
+// process that has a part of the SMs only may hold no cluster of 8 or 16 CTAs
+// of one SM each.
+bool resident_launchable(const cudapic_grid &g, cudaStream_t stream);
 // Enqueues `steps` steps (a positive multiple of n_sub, from the start of an
-// ion cycle).
+// ion cycle); resident_launchable for this stream first.
 int launch_resident(const ResidentArgs &a, const cudapic_grid &g, uint32_t steps, cudaStream_t stream);
 
 }  // namespace cudapic

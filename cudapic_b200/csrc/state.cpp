@@ -375,14 +375,16 @@ constexpr uint64_t RESIDENT_MAX_STEPS = 1000;
 
 // Whether the next steps run in the resident kernel: the driver's default
 // steps of a discharge that fits it, whole ion cycles.
-bool use_resident(const cudapic_state *s, uint64_t n_steps) {
+bool use_resident(cudapic_state *s, uint64_t n_steps) {
     const uint64_t n_sub = s->params.n_sub;
     if (!s->fused || !s->inplace || !s->overlap || !s->solve_ahead || !s->graphs_enabled || s->spawn_collide ||
         s->measure || s->steps_done % n_sub != 0 || n_steps < n_sub || !resident_fits(s->grid, s->params.n_sub))
         return false;
     const void *planes[8] = {s->x[1][0], s->vx[1][0], s->vy[1][0], s->vz[1][0],
                              s->x[1][1], s->vx[1][1], s->vy[1][1], s->vz[1][1]};
-    return electron_step_eligible(planes, 8, s->grid.capacity);
+    if (!electron_step_eligible(planes, 8, s->grid.capacity)) return false;
+    if (s->resident < 0) s->resident = resident_launchable(s->grid, s->stream) ? 1 : 0;
+    return s->resident == 1;
 }
 
 // Enqueues `steps` steps (whole ion cycles) as one launch and moves the
@@ -550,6 +552,7 @@ extern "C" int cudapic_state_set_stream(cudapic_state *s, cudapic_stream_t strea
     if (s->own_stream) cudaStreamDestroy(s->stream);
     s->own_stream = false;
     s->stream = (cudaStream_t)stream;
+    s->resident = -1;
     destroy_graphs(s);
     return CUDAPIC_OK;
 }

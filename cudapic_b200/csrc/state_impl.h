@@ -43,6 +43,9 @@ struct cudapic_state {
     // previous step's samples beside its solve
     float *ef_keep[2] = {};
     bool eepf_pending = false;
+    // whether the resident kernel can be launched into the stream: asked at the
+    // first run that would use it (4 us), -1 until then
+    int resident = -1;
     bool dens_valid = false;  // e_dens[e_cur] and both ion buffers describe the particles
     int graph_key[2][4] = {{-1, -1, -1, -1}, {-1, -1, -1, -1}};  // sides and buffer roles at capture
     float *cs = nullptr, *sigma_tot_e = nullptr, *sigma_tot_i = nullptr;

@@ -175,3 +175,46 @@ def test_uneven_growth_is_shared_out_again(cudapic, cuda_device):
         assert m == ne and np.all((p.x > 0) & (p.x < np.float32(0.025)))
     finally:
         st.close()
+
+
+_FEW_SMS = """
+import sys
+sys.path[:0] = [%r, %r]
+from cuda.bindings import driver as d
+import test_gpu_resident as T
+
+def ok(r):
+    assert r[0] == d.CUresult.CUDA_SUCCESS, r
+    return r[1] if len(r) == 2 else r[1:]
+
+ok(d.cuInit(0))
+dev = ok(d.cuDeviceGet(0))
+ok(d.cuCtxSetCurrent(ok(d.cuDevicePrimaryCtxRetain(dev))))
+sms = ok(d.cuDeviceGetDevResource(dev, d.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+part = ok(d.cuDevSmResourceSplitByCount(1, sms, 0, 32))[0]
+ctx = ok(d.cuGreenCtxCreate(ok(d.cuDevResourceGenerateDesc(part, 1)), dev,
+                            d.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+few = ok(d.cuGreenCtxStreamCreate(ctx, d.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+whole = ok(d.cuStreamCreate(d.CUstream_flags.CU_STREAM_NON_BLOCKING))
+n = 12_000
+st = T._state(T._bulk(n, 1), T._ions(n, 2), 20_000, weight=1e-20, voltage=0.0, pressure=1e-9)  # free flight
+for stream in (few, whole):
+    st.set_stream(int(stream))
+    st.run_steps(20)
+    assert st.counts() == (n, n) and st.device_error() == 0
+st.close()
+print("done")
+"""
+
+
+def test_stream_with_few_sms(cudapic, cuda_device):
+    """A stream of 32 SMs (a green context's) holds no cluster of 16 CTAs of
+    one SM each: the steps run there as launched steps, and on a stream of
+    the whole device as before.  In a process of its own, for the context."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, "-c", _FEW_SMS % (os.path.dirname(here), here)], capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.endswith("done\n"), r.stderr[-2000:]
