@@ -22,6 +22,11 @@ def _state(e, i, capacity, seed=5, **kw):
     return st
 
 
+def _soa(p):
+    from cudapic_b200.sim import ParticlesSoA
+    return ParticlesSoA(*p)
+
+
 def _bulk(n, seed):
     """Electrons of 0.1 to 2 eV in the middle half of the gap.  The vacuum
     field of 250 V and the shot noise of the charge (sqrt(n) W e / (eps0 A))
@@ -173,6 +178,45 @@ def test_uneven_growth_is_shared_out_again(cudapic, cuda_device):
         assert ne == ni and n + 400 < ne < 16_312
         p, m = st.download_electrons()
         assert m == ne and np.all((p.x > 0) & (p.x < np.float32(0.025)))
+    finally:
+        st.close()
+
+
+@pytest.mark.parametrize("launched", [False, True])
+def test_growth_past_a_quarter_in_one_cycle_finds_every_free_slot(cudapic, cuda_device, launched):
+    """A fifth of 5000 electrons are absorbed at once (their slots stay with the
+    first CTAs), the rest have 200 eV and ionize about 0.04 times a step each
+    (50 Pa): 3000 spawns or so per ion cycle, in CTAs without absorbed ones.
+    After the first cycle 2000 to 3000 of the 10 800 slots have not been given
+    out, fewer than the second cycle needs and more than a quarter of the
+    electrons; with the thousand absorbed ones' they suffice.  Nothing gets
+    from the middle fifth of the gap to an electrode in 40 steps, so each
+    ionization leaves one electron and one ion more."""
+    r = np.random.default_rng(21)
+    n, gone = 5000, 1000
+    v = r.normal(0.0, 1.0, (3, n))
+    v *= np.sqrt(2.0 * 200.0 * E_CHARGE / E_MASS) / np.linalg.norm(v, axis=0)
+    x = 0.025 * r.uniform(0.4, 0.6, n)
+    x[:gone], v[0, :gone] = 1e-6, -np.abs(v[0, :gone]) - 1e6
+    e = tuple(a.astype(np.float32) for a in (x, *v))
+    st = _state(e, _ions(n - gone, 22), 10_800, pressure=50.0, weight=1e-6)
+    try:
+        if launched:
+            st.set_overlap(False)
+        first = []
+        for k in (20, 40):  # what the first cycle leaves, then two cycles in one call
+            if k == 40:
+                st.upload_electrons(_soa(e))
+                st.upload_ions(_soa(_ions(n - gone, 22)))
+                st.seed(e_master=(0x1234, 5, 6, 7), i_master=(0x4444, 5, 6, 7))
+            st.run_steps(k)
+            first.append(st.counts())
+        (c1, _), (c2, i2) = first
+        print("\nelectrons after one cycle", c1, "after two", c2)
+        free = 10_800 - (c1 + gone)
+        assert (c1 + gone) // 4 < free < c2 - c1  # the case described
+        assert c2 < 10_800
+        assert st.device_error() == 0 and c2 == i2
     finally:
         st.close()
 
