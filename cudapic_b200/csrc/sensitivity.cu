@@ -1210,7 +1210,7 @@ extern "C" int cudapic_sens_forward(cudapic_sens *s, double voltage, double obs[
     uint32_t c0[C_COUNT] = {s->n_init[0], s->n_init[1], 0, 0, 0, 0, 0, 0};
     CUDAPIC_CHECK(check_cuda(cudaMemcpyAsync(s->cnt, c0, sizeof(c0), cudaMemcpyHostToDevice, st), "sens counters"));
     CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->obs, 0, 2 * sizeof(double), st), "sens obs"));
-    PdlScope pdl(true);
+    PdlScope pdl(s->st->overlap);
     CUDAPIC_CHECK(start_steps(s));
     for (uint32_t t = 0; t < s->K; ++t) {
         if (t % s->S == 0) {
@@ -1248,7 +1248,7 @@ extern "C" int cudapic_sens_backward(cudapic_sens *s, double grad[2]) {
     CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->eb, 0, node_bytes, st), "sens eb"));
     CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->nib_acc, 0, node_bytes, st), "sens nib"));
     CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->vbar, 0, SENS_OBS * sizeof(double), st), "sens vbar"));
-    PdlScope pdl(true);
+    PdlScope pdl(s->st->overlap);
     for (int64_t k = (int64_t)s->n_seg - 1; k >= 0; --k) {
         const uint32_t t0 = (uint32_t)k * s->S;
         if (s->H && (t0 + s->S) % s->H == 0)  // a horizon ends after this segment: the adjoint restarts

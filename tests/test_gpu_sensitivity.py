@@ -92,6 +92,31 @@ def test_forward_sizes_bit_exact(cudapic, cuda_device, oracle, tables, n):
             np.testing.assert_array_equal(got[sp][4][k][:m], ost.rng[sp][k][:m])
 
 
+@pytest.mark.parametrize("on", [True, False])
+def test_launch_overlap_follows_the_state(cudapic, cuda_device, oracle, on):
+    """set_overlap(False): no kernel of a forward and backward run begins
+    before the one before it has ended (by the profiler's record); with it,
+    some do (how many is the host's pace)."""
+    from torch.autograd import DeviceType
+    from torch.profiler import ProfilerActivity, profile
+    from cudapic_b200.sensitivity import VoltageSensitivity
+    st, _, _ = _pair(oracle)
+    st.set_overlap(on)
+    try:
+        with VoltageSensitivity(st, 100, 100) as s:
+            s.forward(V0)
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                s.forward(V0)
+                s.backward()
+    finally:
+        st.close()
+    spans = sorted((e.time_range.start, e.time_range.end) for e in prof.events()
+                   if e.device_type == DeviceType.CUDA and "cudapic" in e.name)
+    assert len(spans) > 1000
+    early = sum(b[0] < a[1] for a, b in zip(spans, spans[1:]))
+    assert early > 0 if on else early == 0, (early, len(spans))
+
+
 def test_adjoint_against_oracle(cudapic, cuda_device, oracle, tables):
     """d obs / dV0 over 200 steps (checkpoints every 40): f32 tangents with
     FP64 field sums on the GPU against the oracle's double adjoint on the
