@@ -901,7 +901,8 @@ struct cudapic_sens {
     uint32_t *spawn_rec = nullptr;
     uint32_t *chunk_count[2] = {nullptr, nullptr};  // spawns per chunk, by the parity of the step
     float *spawn_v = nullptr;
-    float *ckpt = nullptr;               // [n_seg][2][8][cap] (RNG planes stored bitwise)
+    float *ckpt = nullptr;               // [n_seg - 1][2][8][cap] (RNG planes stored bitwise), of segment 1 on:
+                                         // segment 0 starts from init
     uint32_t *ckpt_cnt = nullptr;        // [n_seg][C_COUNT]
     float *tx_e = nullptr, *tv_e = nullptr, *tx_i = nullptr, *tv_i = nullptr, *tE = nullptr;
     uint32_t *tmark = nullptr;           // [S + 1][4]
@@ -1048,6 +1049,11 @@ int copy_planes(cudapic_sens *s, float *dst, const float *src) {
                       "sensitivity plane copy");
 }
 
+// The planes at the start of segment k.
+float *checkpoint_of(const cudapic_sens *s, uint32_t k) {
+    return k ? s->ckpt + (size_t)(k - 1) * 16 * s->cap : s->init[0].x;
+}
+
 // Reverse step t (segment step j).
 int adj_step(cudapic_sens *s, uint32_t t, uint32_t j, const ObsWeights &wP, const ObsWeights &wG) {
     cudaStream_t st = s->stream;
@@ -1137,7 +1143,7 @@ extern "C" int cudapic_sens_create(cudapic_state *st, uint32_t window_steps, uin
         (rc = sens_alloc_t(s, &s->spawn_rec, cap)) || (rc = sens_alloc_t(s, &s->spawn_v, 6 * cap)) ||
         (rc = sens_alloc_t(s, &s->chunk_count[0], cap / SENS_CHUNK + 2)) ||
         (rc = sens_alloc_t(s, &s->chunk_count[1], cap / SENS_CHUNK + 2)) ||
-        (rc = sens_alloc_t(s, &s->ckpt, (size_t)s->n_seg * 16 * cap)) ||
+        (rc = sens_alloc_t(s, &s->ckpt, (size_t)(s->n_seg - 1) * 16 * cap)) ||
         (rc = sens_alloc_t(s, &s->ckpt_cnt, (size_t)s->n_seg * C_COUNT)) ||
         (rc = sens_alloc_t(s, &s->tx_e, (size_t)s->S * cap)) || (rc = sens_alloc_t(s, &s->tv_e, (size_t)s->S * cap)) ||
         (rc = sens_alloc_t(s, &s->tx_i, (size_t)(s->S / s->n_sub) * cap)) ||
@@ -1215,7 +1221,7 @@ extern "C" int cudapic_sens_forward(cudapic_sens *s, double voltage, double obs[
     for (uint32_t t = 0; t < s->K; ++t) {
         if (t % s->S == 0) {
             const uint32_t k = t / s->S;
-            CUDAPIC_CHECK(copy_planes(s, s->ckpt + (size_t)k * 16 * cap, s->cur[0].x));
+            if (k) CUDAPIC_CHECK(copy_planes(s, checkpoint_of(s, k), s->cur[0].x));
             CUDAPIC_CHECK(check_cuda(cudaMemcpyAsync(s->ckpt_cnt + (size_t)k * C_COUNT, s->cnt, sizeof(uint32_t) * C_COUNT,
                                                      cudaMemcpyDeviceToDevice, st), "sens checkpoint counters"));
         }
@@ -1254,7 +1260,7 @@ extern "C" int cudapic_sens_backward(cudapic_sens *s, double grad[2]) {
         if (s->H && (t0 + s->S) % s->H == 0)  // a horizon ends after this segment: the adjoint restarts
             CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->adj, 0, adj_bytes, st), "sens horizon"));
         // recompute the segment from its checkpoint, recording the tape
-        CUDAPIC_CHECK(copy_planes(s, s->cur[0].x, s->ckpt + (size_t)k * 16 * cap));
+        CUDAPIC_CHECK(copy_planes(s, s->cur[0].x, checkpoint_of(s, (uint32_t)k)));
         CUDAPIC_CHECK(check_cuda(cudaMemcpyAsync(s->cnt, s->ckpt_cnt + (size_t)k * C_COUNT, sizeof(uint32_t) * C_COUNT,
                                                  cudaMemcpyDeviceToDevice, st), "sens restore counters"));
         CUDAPIC_CHECK(check_cuda(cudaMemsetAsync(s->cnt + C_REC_E, 0, 2 * sizeof(uint32_t), st), "sens records"));

@@ -92,6 +92,29 @@ def test_forward_sizes_bit_exact(cudapic, cuda_device, oracle, tables, n):
             np.testing.assert_array_equal(got[sp][4][k][:m], ost.rng[sp][k][:m])
 
 
+@pytest.mark.parametrize("window,every", [(100, 100), (200, 40)])
+def test_device_memory(cudapic, cuda_device, oracle, window, every):
+    """Per slot: initial and present state 64 B each, spawn requests 28, a
+    checkpoint of 64 per interval, the tape's 8 per step and per ion step,
+    adjoints of one observable 32 (two are held: the first checkpoint is the
+    initial state); the records of 36 and 40 B; nodes of the tape; 64 KB of
+    small buffers."""
+    from cudapic_b200.sensitivity import VoltageSensitivity
+    st, _, _ = _pair(oracle, n=20_000)
+    cap = st.capacity
+    try:
+        with VoltageSensitivity(st, window, every) as s:
+            got = s.info()["device_bytes"]
+            s.forward(V0)
+            s.backward()
+            assert s.info()["device_bytes"] == got
+    finally:
+        st.close()
+    slot = 64 + 64 + 28 + 64 * (window // every) + 8 * every + 8 * (every // 20) + 32
+    records = 36 * (cap * every // 32 + 65536) + 40 * (cap * (every // 20) // 8 + 65536)
+    assert got <= slot * cap + records + 4 * 400 * every + 65536
+
+
 @pytest.mark.parametrize("on", [True, False])
 def test_launch_overlap_follows_the_state(cudapic, cuda_device, oracle, on):
     """set_overlap(False): no kernel of a forward and backward run begins
