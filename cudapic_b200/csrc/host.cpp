@@ -384,6 +384,16 @@ void cs_range(double gas_density, float *cs, float *se, float *si, uint32_t lo, 
 
 }  // namespace
 
+namespace cudapic {
+float ionization_from(const float *cs) {
+    const float *ion = cs + 2 * (size_t)CUDAPIC_CS_RANGES;
+    uint32_t first = 0;
+    while (first < CUDAPIC_CS_RANGES && ion[first] == 0.0f) ++first;
+    // entry (uint32)(E / 0.001 + 0.5) is below `first` for E < 0.001 (first - 1)
+    return first > 1 ? (float)(0.001 * (double)(first - 1)) : 0.0f;
+}
+}  // namespace cudapic
+
 extern "C" int cudapic_cross_sections(double gas_density, float *cs, float *sigma_tot_e, float *sigma_tot_i) {
     if (!cs || !sigma_tot_e || !sigma_tot_i) return fail(CUDAPIC_ERR_ARG, "cross_sections: null pointer");
     if (!(gas_density > 0)) return fail(CUDAPIC_ERR_ARG, "cross_sections: gas density must be positive");

@@ -189,8 +189,12 @@ enum XtRaw : int {
 // Adds one species' particles (before the push) to the XT column of the step
 // the Poisson kernel just solved.
 int launch_xt_particles(bool ions, const float *x, const float *vx, const float *vy, const float *vz,
-                        const uint32_t *n_active, const float *efield, const float *cs, const uint32_t *step_counter,
-                        const cudapic_grid &g, uint32_t n_xt, double *xt, cudaStream_t stream);
+                        const uint32_t *n_active, const float *efield, const float *cs, float ion_from,
+                        const uint32_t *step_counter, const cudapic_grid &g, uint32_t n_xt, double *xt,
+                        cudaStream_t stream);
+// An energy [eV] below which every entry of the ionization table cs[2] that
+// an electron can meet is zero (XT's ionization rate skips the table there).
+float ionization_from(const float *cs);
 // Largest electron / ion collision frequencies of the total tables [1/s]
 // (C/eduPIC.cc:252-276) and the CFL energy limit [eV] (report.cpp).
 void table_coll_freqs(const float *sigma_tot_e, const float *sigma_tot_i, double *max_e, double *max_i);

@@ -21,7 +21,7 @@
 // non-empty node to the FP64 column with one global atomic, so the long
 // accumulation is FP64 while the per-step partial sums are f32.  Bound by the
 // shared f32 atomics (eight per electron; the two of the ionization rate only
-// above the threshold, below which the table is zero) and by latency: with
+// from the energy of its table's first entry on) and by latency: with
 // 512 threads and one particle per thread and round, every round waiting for
 // its loads, 400 000 electrons took 15.9 us, now 11.3 us (alone).
 // The grid quantities are added by the solve's launch (kernels_poisson.cu).
@@ -38,8 +38,6 @@ namespace cudapic {
 namespace {
 
 constexpr int XT_THREADS = 1024;
-// Below this energy the ionization table is zero (threshold 15.8 eV)
-constexpr float XT_NO_IONIZATION_EV = 15.7f;
 
 // Column of the step just solved: the Poisson kernel advanced the step counter.
 __device__ __forceinline__ uint32_t xt_column(const uint32_t *step_counter, uint32_t n_t) {
@@ -48,12 +46,14 @@ __device__ __forceinline__ uint32_t xt_column(const uint32_t *step_counter, uint
 }
 
 // Adds the particles [lo, hi) of the planes (16-byte aligned, their capacity
-// a multiple of 4) to the CTA's shared histograms h[q * n_g + node].
+// a multiple of 4) to the CTA's shared histograms h[q * n_g + node]; cs_ion is
+// zero for energies below ion_from [eV] (ionization_from).
 template <bool ION>
 __device__ __forceinline__ void xt_accumulate(const float *__restrict__ x, const float *__restrict__ vx,
                                               const float *__restrict__ vy, const float *__restrict__ vz,
                                               uint32_t lo, uint32_t hi, const float *__restrict__ ef,
-                                              const float *__restrict__ cs_ion, const cudapic_grid &g, float *h) {
+                                              const float *__restrict__ cs_ion, float ion_from, const cudapic_grid &g,
+                                              float *h) {
     const uint32_t n_g = g.n_g;
     const float inv_dx = g.inv_dx;
     const float factor = ION ? g.factor_i : g.factor_e;
@@ -82,7 +82,7 @@ __device__ __forceinline__ void xt_accumulate(const float *__restrict__ x, const
             atomicAdd(&h[n_g + p + 1], c2 * v);
             atomicAdd(&h[2 * n_g + p], c1 * energy);
             atomicAdd(&h[2 * n_g + p + 1], c2 * energy);
-            if (!ION && !(energy < XT_NO_IONIZATION_EV)) {
+            if (!ION && !(energy < ion_from)) {
                 const float t = fminf(energy / DE_CS_F + 0.5f, (float)(CS_RANGES - 1));
                 const float rate = __ldg(cs_ion + (uint32_t)t) * sqrtf(v2) * rate_scale;
                 atomicAdd(&h[3 * n_g + p], c1 * rate);
@@ -118,7 +118,7 @@ template <bool ION>
 __global__ void __launch_bounds__(XT_THREADS)
     xt_particles_kernel(const float *__restrict__ x, const float *__restrict__ vx, const float *__restrict__ vy,
                         const float *__restrict__ vz, const uint32_t *__restrict__ n_active,
-                        const float *__restrict__ efield, const float *__restrict__ cs,
+                        const float *__restrict__ efield, const float *__restrict__ cs, float ion_from,
                         const uint32_t *__restrict__ step_counter, const __grid_constant__ cudapic_grid g, uint32_t n_xt,
                         double *xt) {
     extern __shared__ float xt_h[];  // [Q][n_g]
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(XT_THREADS)
     const uint32_t col = xt_column(step_counter, g.n_t);
     const uint32_t chunk = ((n + gridDim.x - 1) / gridDim.x + 3u) & ~3u;
     const uint32_t lo = min(n, blockIdx.x * chunk), hi = min(n, lo + chunk);
-    xt_accumulate<ION>(x, vx, vy, vz, lo, hi, efield, cs + 2 * CS_RANGES, g, xt_h);
+    xt_accumulate<ION>(x, vx, vy, vz, lo, hi, efield, cs + 2 * CS_RANGES, ion_from, g, xt_h);
     xt_flush(xt_h, Q, xt, ION ? XT_COUNT_I : XT_COUNT_E, g.n_g, n_xt, col);
 }
 
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(XT_THREADS)
         for (uint32_t k = threadIdx.x; k < Q * n_g; k += blockDim.x) bxt_h[k] = 0.0f;
         __syncthreads();
         xt_accumulate<ION>(sp.x + dd.off, sp.vx + dd.off, sp.vy + dd.off, sp.vz + dd.off, a - pfx[d], b - pfx[d],
-                           dd.efield, dd.cs + 2 * CS_RANGES, dd.g, bxt_h);
+                           dd.efield, dd.cs + 2 * CS_RANGES, dd.ion_from, dd.g, bxt_h);
         xt_flush(bxt_h, Q, dd.xt, ION ? XT_COUNT_I : XT_COUNT_E, n_g, dd.n_xt, xt_column(dd.counters + 3, dd.g.n_t));
     }
 }
@@ -190,8 +190,9 @@ __global__ void __launch_bounds__(XT_THREADS)
 }  // namespace
 
 int launch_xt_particles(bool ions, const float *x, const float *vx, const float *vy, const float *vz,
-                        const uint32_t *n_active, const float *efield, const float *cs, const uint32_t *step_counter,
-                        const cudapic_grid &g, uint32_t n_xt, double *xt, cudaStream_t stream) {
+                        const uint32_t *n_active, const float *efield, const float *cs, float ion_from,
+                        const uint32_t *step_counter, const cudapic_grid &g, uint32_t n_xt, double *xt,
+                        cudaStream_t stream) {
     const size_t need = (size_t)(ions ? 3 : 4) * g.n_g * sizeof(float);
     if (need > (size_t)max_smem_optin()) return fail(CUDAPIC_ERR_ARG, "xt: n_g too large");
     // at least half of an SM's shared memory, so that no SM takes two CTAs:
@@ -204,7 +205,7 @@ int launch_xt_particles(bool ions, const float *x, const float *vx, const float 
     CUDAPIC_CHECK(kernel_smem((const void *)kern, smem, "xt"));
     const unsigned grid = persistent_grid(1, ((uint64_t)g.capacity + XT_THREADS - 1) / XT_THREADS);
     return launch_kernel(ions ? "xt_ions" : "xt_electrons", kern, dim3(grid), dim3(XT_THREADS), smem, stream, x, vx,
-                         vy, vz, n_active, efield, cs, step_counter, g, n_xt, xt);
+                         vy, vz, n_active, efield, cs, ion_from, step_counter, g, n_xt, xt);
 }
 
 int launch_batch_xt_particles(bool ions, const SidePlanes &sp, const BatchDisc *desc, uint32_t D, uint32_t max_n_g,

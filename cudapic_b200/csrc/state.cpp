@@ -273,11 +273,11 @@ int enqueue_step(cudapic_state *s, bool ion_step, bool compact, int next_ion) {
     if (s->measure) {
         if (s->xt) {  // XT diagnostics: the particles before their push
             CUDAPIC_CHECK(launch_xt_particles(false, s->x[E][se], s->vx[E][se], s->vy[E][se], s->vz[E][se], s->n_e(),
-                                              s->efield, s->cs, s->step_counter(), g, s->n_xt, s->xt, st));
+                                              s->efield, s->cs, s->ion_from, s->step_counter(), g, s->n_xt, s->xt, st));
             if (ion_step)
                 CUDAPIC_CHECK(launch_xt_particles(true, s->x[I][si], s->vx[I][si], s->vy[I][si], s->vz[I][si],
-                                                  s->n_i(), s->efield, s->cs, s->step_counter(), g, s->n_xt, s->xt,
-                                                  st));
+                                                  s->n_i(), s->efield, s->cs, s->ion_from, s->step_counter(), g,
+                                                  s->n_xt, s->xt, st));
         }
     }
     if (fused) {
@@ -519,6 +519,7 @@ extern "C" int cudapic_state_create(const cudapic_params *p, int device, cudapic
     if ((rc = cudapic_cross_sections(grid.gas_density, cs.data(), se.data(), si.data()))) return cleanup(rc);
     s->sigma_max_e = *std::max_element(se.begin(), se.end());
     s->ion_k = ion_reject_k(*std::max_element(si.begin(), si.end()), s->grid);
+    s->ion_from = ionization_from(cs.data());
     table_coll_freqs(se.data(), si.data(), &s->max_e_coll_freq, &s->max_i_coll_freq);
     if ((rc = check_cuda(cudaMemcpyAsync(s->pot0_table, table.data(), table.size() * sizeof(float),
                                          cudaMemcpyHostToDevice, s->stream), "upload pot0 table")) ||

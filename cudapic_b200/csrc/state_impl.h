@@ -51,6 +51,7 @@ struct cudapic_state {
     float *cs = nullptr, *sigma_tot_e = nullptr, *sigma_tot_i = nullptr;
     float sigma_max_e = 0.0f;  // largest entry of sigma_tot_e (the fused step's certain-rejection bound)
     float ion_k = INFINITY;    // the fused driver's ion-test bound (ion_reject_k of sigma_tot_i)
+    float ion_from = 0.0f;     // no ionization below this energy (ionization_from of cs)
     double *cumul_e = nullptr, *cumul_i = nullptr;
     cudapic_wall_counters *wall = nullptr;  // [0] electrons, [1] ions (measurement window)
     // measurement window: [0] electron and [1] ion collision events, [2] EEPF

@@ -99,3 +99,25 @@ def test_bound_without_the_root_is_the_stricter_one(cudapic, oracle, tables, n_t
         assert np.all(near[passes(near)] >= b[passes(near)])
     if n_t == 4000:
         assert passes(u).mean() > 0.9
+
+
+@pytest.mark.parametrize("first", [None, 0, 1, 2, 11, 5001, 15801, 999_999])
+def test_xt_ionization_bound_follows_the_table(cudapic, tables, first):
+    """The energy below which the XT pass skips the ionization table
+    (ionization_from) comes from the table itself: no entry that an electron
+    below it meets (f32 index of common.cuh) has ionization in it, and the
+    next two energies' may."""
+    import ctypes
+    lib = cudapic.lib
+    fn = lib._ZN7cudapic15ionization_fromEPKf
+    fn.restype, fn.argtypes = ctypes.c_float, [ctypes.c_void_p]
+    cs = np.ascontiguousarray(tables[0]).reshape(5, -1).copy()
+    if first is not None:
+        cs[2, :first], cs[2, first:] = 0.0, 1e-20
+    start = int(np.argmax(cs[2] != 0.0))
+    assert first is None or start == first
+    e = np.float32(fn(cs.ctypes.data))
+    index = lambda v: int(np.float32(np.float32(v) / np.float32(0.001)) + np.float32(0.5))  # noqa: E731
+    if e > 0:
+        assert index(np.nextafter(e, np.float32(0))) < max(start, 1)
+    assert start <= index(e) + 2
