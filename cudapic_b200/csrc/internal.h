@@ -44,6 +44,8 @@ int validate_grid(const cudapic_grid *g);
 
 // Current launch shapes (defaults filled in for zero fields).
 cudapic_tuning tuning();
+// Rounds prefetched by the in-place stream pass of one discharge or a batch.
+uint32_t prefetch_rounds(const cudapic_tuning &t, bool batch);
 // Advanced by every cudapic_set_tuning: captured graphs baked the shapes of
 // the generation they were captured in.
 uint64_t tuning_generation();

@@ -661,7 +661,7 @@ int launch_batch_inplace(const InplacePlanes &pl, const CollList &list, const Ba
     const uint32_t per_round = copies ? (uint32_t)((IP_WARPS + copies - 1) / copies) * 32u * IP_ROW : 1u;
     const uint32_t epoch = copies ? std::max(1u, DEP_MAX_PER_COPY / per_round) : 0xffffffffu;
     return launch_kernel("batch_inplace_electrons", kern, dim3(grid), dim3(IP_THREADS), bytes(), stream, pl, list,
-                         desc, counts, D, r.dens, ef_pad, copies, epoch, (uint32_t)std::max(t.inplace_prefetch ? t.inplace_prefetch : 1, 0),
+                         desc, counts, D, r.dens, ef_pad, copies, epoch, prefetch_rounds(t, true),
                          r.dens);  // the role turns every step, and the direction with it
 }
 

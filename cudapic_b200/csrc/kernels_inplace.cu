@@ -199,14 +199,10 @@ int launch_electron_inplace(const InplacePlanes &pl, const float *efield, const 
     // rounds per deposit drain: a copy receives ceil(WARPS / copies) warps x 32 lanes x IP_ROW slots per round
     const uint32_t per_round = copies ? (uint32_t)((IP_WARPS + copies - 1) / copies) * 32u * IP_ROW : 1u;
     const uint32_t epoch = copies ? std::max(1u, DEP_MAX_PER_COPY / per_round) : 0xffffffffu;
-    // no prefetch unless asked for: where the CTAs stream through one window
-    // of the planes, one round ahead is 4 to 8 % slower (8.4 M electrons in
-    // the driver 124 us per step, without 115); a batch's CTAs, each in its
-    // own share, gain 3 % by it
     return launch_kernel("step_electrons_inplace", kern, dim3(grid), dim3(IP_THREADS),
                          inplace_smem_bytes(copies, ef_pad), stream, pl, efield, sigma_tot_e, cs, sigma_max, n_active, list,
                          count, dens_e, g, ef_pad, copies, epoch, wall, spawn_from,
-                         (uint32_t)std::max(t.inplace_prefetch, 0), (int)reverse);
+                         prefetch_rounds(t, false), (int)reverse);
 }
 
 int launch_electron_scatter(const InplacePlanes &pl, const CollList &list, const float *cs, uint32_t *count,
