@@ -221,6 +221,134 @@ def test_growth_past_a_quarter_in_one_cycle_finds_every_free_slot(cudapic, cuda_
         st.close()
 
 
+def _free(n, seed, n_sub=20, capacity=16_312, voltage=250.0, speed=2e5, **kw):
+    """A state whose electrons and ions only fall through the vacuum field: no
+    gas, no charge.  No draw and no slot then decides anything, so two paths
+    give the same particles bit for bit whatever slots these end in."""
+    r = np.random.default_rng(seed)
+    x = (0.025 * r.uniform(0.1, 0.9, (2, n))).astype(np.float32)
+    v = (r.normal(0.0, 1.0, (2, 3, n)) * np.array([[[speed]], [[300.0]]])).astype(np.float32)
+    st = _state((x[0], *v[0]), (x[1], *v[1]), capacity, seed=seed, n_sub=n_sub, voltage=voltage, pressure=1e-9,
+                weight=1e-20, **kw)
+    return st
+
+
+def _particles(st):
+    """Rows of both species in the order of vy, vz, which nothing changes."""
+    out = []
+    for soa, n in (st.download_electrons(), st.download_ions()):
+        rows = np.stack([soa.x, soa.vx, soa.vy, soa.vz])[:, :n]
+        out.append(rows[:, np.lexsort((rows[3], rows[2]))])
+    assert st.device_error() == 0
+    return out
+
+
+@pytest.mark.parametrize("n,capacity,n_sub,calls", [
+    (2047, 4096, 2, (40, 1, 139)), (5003, 16_312, 8, (24, 3, 37, 64)), (5003, 16_312, 20, (7, 133)),
+    (20_001, 32_688, 20, (20,) * 6), (9001, 9004, 50, (120, 30))])
+def test_rows_match_launched_steps(cudapic, cuda_device, n, capacity, n_sub, calls):
+    """Several N_SUB, calls that begin or end inside an ion cycle, many short
+    ones: each electron's and ion's whole row as the launched steps give it,
+    with the field's acceleration and absorption at the electrodes."""
+    got = []
+    for launched in (False, True):
+        st = _free(n, 31, n_sub, capacity)
+        try:
+            if launched:
+                st.set_overlap(False)
+            for c in calls:
+                st.run_steps(c)
+            assert st.steps_done() == sum(calls)
+            got.append(_particles(st))
+        finally:
+            st.close()
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
+    assert 0 < got[0][0].shape[1] < n  # some electrons reached an electrode
+
+
+def test_two_states_on_two_streams(cudapic, cuda_device):
+    """Two discharges enqueued in turn without waiting: each as when alone."""
+    want = []
+    for seed, n in ((41, 3001), (42, 15_001)):
+        with _free(n, seed) as st:
+            st.set_overlap(False)
+            st.run_steps(200)
+            want.append(_particles(st))
+    both = [_free(3001, 41), _free(15_001, 42)]
+    try:
+        for _ in range(5):
+            for st in both:
+                st.run_steps(40)
+        for st, w in zip(both, want):
+            for a, b in zip(_particles(st), w):
+                np.testing.assert_array_equal(a, b)
+    finally:
+        for st in both:
+            st.close()
+
+
+def test_checkpoint_of_a_resident_run(cudapic, cuda_device, tmp_path):
+    """One RF cycle, saved, loaded into another state: the RNG planes are the
+    same, and 40 more steps give the same particles and planes in both."""
+    from gpu_util import device_array
+    planes = lambda st: [device_array(p, st.capacity, np.uint32) for sp in (0, 1) for p in st.buffers().rng[sp]]  # noqa: E731
+    a, b = (_free(4001, 51, voltage=0.0, speed=5e3) for _ in range(2))
+    try:
+        a.run_steps(4000)
+        a.save(tmp_path / "picdata.bin")
+        b.load(tmp_path / "picdata.bin")
+        for steps in (0, 40):
+            for st in (a, b):
+                if steps:
+                    st.run_steps(steps)
+                st.synchronize()
+            for p, q in zip(planes(a), planes(b)):
+                np.testing.assert_array_equal(p, q)
+        for p, q in zip(_particles(a), _particles(b)):
+            np.testing.assert_array_equal(p, q)
+    finally:
+        a.close()
+        b.close()
+
+
+def test_overflow_leaves_counters_planes_and_densities_in_agreement(cudapic, cuda_device, oracle):
+    """Spawns into full planes, as test_capacity_overflow_is_flagged, by what
+    the device holds: both counters within the capacity, every slot below them
+    a particle of its own in the gap, and the densities those of just these
+    particles (2e-5, as the deposit elsewhere)."""
+    from gpu_util import device_array
+    r = np.random.default_rng(3)
+    n, w = 4000, 10.0
+    v = r.normal(0.0, 1.0, (3, n))
+    v *= np.sqrt(2.0 * 60.0 * E_CHARGE / E_MASS) / np.linalg.norm(v, axis=0)
+    e = tuple(a.astype(np.float32) for a in (0.025 * r.uniform(0.4, 0.6, n), *v))
+    st = _state(e, _ions(n, 4), n + 4, pressure=50.0, weight=w)
+    ph = oracle.phys_from_params(capacity=n + 4, weight=w)
+    try:
+        st.run_steps(200)
+        st.synchronize()
+        b = st.buffers()
+        raw = [int(device_array(p, 1, np.uint32)[0]) for p in (b.n_electrons, b.n_ions)]
+        assert max(raw) <= n + 4 and raw == list(st.counts()) and raw[1] == n + 4
+        parts = []
+        for sp, m in enumerate(raw):
+            rows = np.stack([device_array(p[sp], m, np.float32) for p in (b.x, b.vx, b.vy, b.vz)])
+            assert np.all(np.isfinite(rows)) and np.all((rows[0] >= 0) & (rows[0] <= np.float32(0.025)))
+            assert np.unique(rows, axis=1).shape[1] == m
+            parts.append(rows[0])
+        dens = device_array(b.e_density, 400, np.float32)
+        ref = oracle.get_density_f64(parts[0], ph)
+        assert np.linalg.norm(dens - ref) <= 2e-5 * np.linalg.norm(ref)
+        st.run_steps(1)  # an ion step: the density collected over the cycle becomes current
+        st.synchronize()
+        dens = device_array(st.buffers().i_density, 400, np.float32)
+        ref = oracle.get_density_f64(parts[1], ph)
+        assert np.linalg.norm(dens - ref) <= 2e-5 * np.linalg.norm(ref)
+    finally:
+        st.close()
+
+
 _FEW_SMS = """
 import sys
 sys.path[:0] = [%r, %r]
