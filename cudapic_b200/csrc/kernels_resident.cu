@@ -31,9 +31,9 @@
 // counters, densities and RNG planes are left as the driver's own steps leave
 // them, so runs may mix both.
 // Measured (N_G = 400, reference discharge; us per step alone / per step with
-// three discharges in flight), here against the launched steps: 1000
-// electrons 4.8 / 1.6 against 12.5 / 4.3, 12 300 electrons 6.7 / 2.2 against
-// 13.4 / 4.5, 24 200 electrons (16 CTAs) 7.6 / 2.6 against 13.9 / 4.8.  What is
+// three discharges in flight), here against the launched steps: 1300
+// electrons 5.4 / 1.8 against 10.0 / 3.9, 13 700 electrons 6.5 / 2.2 against
+// 11.3 / 4.2, 27 500 electrons (16 CTAs) 7.7 / 2.6 against 12.4 / 4.3.  What is
 // left is latency: reading the peers' sums (0.6 us), the barrier with the
 // wait for the slowest CTA (1 us), one chain of scattering (1 us), the solve.
 #include <cooperative_groups.h>
@@ -711,10 +711,11 @@ __global__ void __launch_bounds__(RS_THREADS, 1)
 namespace {
 
 // CTAs of the cluster for a capacity (0: none fits): a share-out never fills
-// more than RS_FILL entries (shares are rounded up to 4 slots).  Larger
-// discharges fill enough SMs for the launched steps to take over (with the
-// electrons in global memory this kernel took 17 us per step at 48 000
-// electrons, the launched steps 13.7).
+// more than RS_FILL entries (shares are rounded up to 4 slots).  The capacity
+// counts and not the population, which may grow to it inside the kernel.  The
+// line is the room of the largest cluster and not where the launched steps get
+// faster: 27 500 electrons in 32 688 slots take 7.7 us per step (2.6 with three
+// discharges in flight), launched, in 32 692 slots, 12.4 (4.3).
 int resident_cluster(const cudapic_grid &g) {
     const uint64_t need = (uint64_t)g.capacity + 64;
     return need <= 8 * RS_FILL ? 8 : need <= 16 * RS_FILL ? 16 : 0;

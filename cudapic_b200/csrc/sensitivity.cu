@@ -345,7 +345,7 @@ __device__ __forceinline__ void deposit_spawn(unsigned long long *hist, float x,
 // The field of a step, one CTA: marks the slot and record counts at the
 // step's start (mark may be null) and the spawn bases, turns the node sums
 // into f32 densities (boundary nodes doubled) and clears them, and solves
-// with the drivers' two-scan arithmetic (poisson_body), which the recompute
+// by two scans (poisson_body; the drivers solve by one), which the recompute
 // and the oracle's model repeat bit for bit.  efield: the step's field (on
 // the tape when recording).
 template <int PT>
