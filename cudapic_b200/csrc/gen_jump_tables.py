@@ -11,7 +11,8 @@ import sys
 
 JUMP = (0x8764000B, 0xF542D2D3, 0x6FA035C3, 0x77F2DB5B)
 M32 = 0xFFFFFFFF
-LEVELS = 28       # level b is J^(2^b): up to 2^28 streams
+FIRST_LEVEL = 0   # level b of the table is J^(2^(b + FIRST_LEVEL))
+LEVELS = 28       # levels 0..27: up to 2^28 streams
 
 
 def _next(s):
