@@ -8,7 +8,10 @@ check_collisions_e, check_collisions_e_deposit, check_collisions_i (and
 check_collisions_i_bounded, the drivers' entry given max(sigma_tot_i)) and
 step_electrons (the *_deposit variants also deposit the next step's density;
 step_electrons is the fused driver's compacting electron kernel,
-step_electrons_inplace the stream pass of its in-place step).  Prints one JSON line with the median time, the particle
+step_electrons_inplace the stream pass of its in-place step).  memory_inplace
+is none of them: a plain in-place add over as many bytes per particle as the
+stream pass moves (each line read and written back), what the memory itself
+gives such a pass.  Prints one JSON line with the median time, the particle
 count and the algorithmic bytes per launch.
 """
 import argparse
@@ -18,7 +21,7 @@ import statistics
 BYTES = {"get_density": 4, "move_and_compact": 32, "move_and_compact_deposit": 32, "check_collisions_e": 44,
          "check_collisions_e_deposit": 44, "check_collisions_i": 44, "check_collisions_i_bounded": 44,
          "solve_poisson": 0, "step_electrons": 64,
-         "step_electrons_inplace": 56}
+         "step_electrons_inplace": 56, "memory_inplace": 56}
 
 
 def main():
@@ -55,6 +58,7 @@ def main():
     ef = torch.zeros(g.n_g, dtype=torch.float32, device="cuda")
     alive = u32(0)
     ccount = u32(0)
+    plane = torch.zeros(BYTES["memory_inplace"] // 8 * n_e, dtype=torch.float32, device="cuda")
     sigma_max_i = float(K.init_cross_sections(g.gas_density)[2].max())  # the ion table's largest entry
     fns = {
         "get_density": (lambda: K.get_density(b.x[0], dens, ne_c, g, stream=s), lambda: dens.zero_(), n_e),
@@ -88,6 +92,7 @@ def main():
             b.efield, b.x[0], b.vx[0], b.vy[0], b.vz[0], *b.rng[0], b.sigma_tot_e, b.cs, b.sigma_max_e, ne_c,
             (b.tmp_x[0], b.tmp_vx[0], b.tmp_vy[0], b.tmp_vz[0], b.tmp_x[1], b.tmp_vx[1], b.tmp_vy[1], b.tmp_vz[1]),
             ccount, dens, g, stream=s), lambda: (ccount.zero_(), dens.zero_()), n_e),
+        "memory_inplace": (lambda: plane.add_(1.0), None, n_e),
     }
     fn, pre, n = fns[a.kernel]
     if a.tuning:

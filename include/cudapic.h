@@ -488,7 +488,8 @@ int cudapic_state_set_measure(cudapic_state *s, int on);
  * on the state's stream.  Asynchronous.  With every switch below at its default,
  * not measuring, a capacity of at most 32 688 and N_G <= 1024, whole ion cycles
  * (N_SUB steps from a multiple of N_SUB on) run in one launch of one
- * thread-block cluster, with the same steps and the electrons compact at the
+ * thread-block cluster of 8 or 16 CTAs, an SM each, where the stream's share
+ * of the GPU holds one, with the same steps and the electrons compact at the
  * end of every cycle; the rest of a run, and every other state, in the
  * launches described below. */
 int cudapic_state_run_steps(cudapic_state *s, uint64_t n_steps);
@@ -527,7 +528,8 @@ int cudapic_state_set_spawn_collide(cudapic_state *s, int on);
 int cudapic_state_set_solve_ahead(cudapic_state *s, int on);
 /* on (default): the driver launches its kernels with programmatic dependent
  * launch, so a kernel's launch and prologue overlap the previous kernel's
- * tail (every kernel waits for its predecessor before touching global data).
+ * tail (every kernel waits for its predecessor before touching global data),
+ * and so do sensitivities made from this state.
  * off: plain stream order.  The captured graphs are rebuilt. */
 int cudapic_state_set_overlap(cudapic_state *s, int on);
 /* on (default when N_T is a multiple of N_SUB): run_steps replays captured
