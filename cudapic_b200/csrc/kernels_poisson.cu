@@ -81,6 +81,35 @@ struct MeasureGrid {
         }
     }
 };
+
+// Beyond this many nodes one CTA takes longer over the grid quantities (each XT
+// sum is a sector of its own: 12 doubles read and written per node through one
+// SM) than a further launch of a few CTAs costs.  A measured step of 3000
+// particles takes, by the solve's CTA / by a launch behind it, 21.7 / 23.5 us at
+// 400 nodes, 24.6 / 24.3 at 800, 25.9 / 24.3 at 1024, 45.8 / 28.1 at 4096; of
+// 400 000 34.4 / 37.1, 38.1 / 38.9, 39.7 / 38.2 and 65.9 / 44.4.
+constexpr uint32_t MEASURE_GRID_MAX = 800;
+
+// The same for larger grids, behind the solve (the step counter is past the
+// step): one node per thread.
+__global__ void __launch_bounds__(256)
+    measure_grid_kernel(const float *__restrict__ e_density, const float *__restrict__ i_density,
+                        const float *__restrict__ pot, const float *__restrict__ efield,
+                        const uint32_t *__restrict__ step_counter, const __grid_constant__ cudapic_grid g,
+                        const PoissonMeasure m) {
+    grid_dep_wait();
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= g.n_g) return;
+    const uint32_t col = (*step_counter + g.n_t - 1u) % g.n_t / XT_BIN;
+    const float v[4] = {pot[k], efield[k], e_density[k], i_density[k]};
+    if (m.ef_keep) m.ef_keep[k] = v[1];
+    m.cumul_e[k] += (double)v[2];
+    if (m.cumul_i) m.cumul_i[k] += (double)v[3];
+    if (!m.xt) return;
+    const size_t plane = (size_t)g.n_g * m.n_xt, at = (size_t)k * m.n_xt + col;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) m.xt[(XT_POT + q) * plane + at] += (double)v[q];
+}
 static_assert(XT_EFIELD == XT_POT + 1 && XT_NE == XT_POT + 2 && XT_NI == XT_POT + 3, "order of the grid quantities");
 
 template <typename T, int PT>
@@ -463,9 +492,14 @@ int launch_poisson(const float *e_density, const float *i_density, float *pot, f
                    const EepfSamples *eepf) {
     if (g.n_g > (uint32_t)(POIS_MAX_THREADS * POIS_MAX_PER_THREAD))
         return fail(CUDAPIC_ERR_ARG, "solve_poisson: n_g > 16384");
-    if (g.flags & CUDAPIC_FLAG_POISSON_F32_SCAN)
-        return launch_poisson_pt<float>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, stream, zero_a, zero_b, meas, eepf);
-    return launch_poisson_pt<double>(e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, stream, zero_a, zero_b, meas, eepf);
+    const bool behind = meas.cumul_e && g.n_g > MEASURE_GRID_MAX;
+    const PoissonMeasure in = behind ? PoissonMeasure{} : meas;
+    const bool f32 = (g.flags & CUDAPIC_FLAG_POISSON_F32_SCAN) != 0;
+    CUDAPIC_CHECK((f32 ? launch_poisson_pt<float> : launch_poisson_pt<double>)(
+        e_density, i_density, pot, efield, pot0, pot0_table, step_counter, g, stream, zero_a, zero_b, in, eepf));
+    if (!behind) return CUDAPIC_OK;
+    return launch_kernel("measure_grid", measure_grid_kernel, dim3((g.n_g + 255) / 256), dim3(256), 0, stream, e_density,
+                         i_density, (const float *)pot, (const float *)efield, (const uint32_t *)step_counter, g, meas);
 }
 
 // Batched solve: CTA d solves discharge d of the batch (the driver variant

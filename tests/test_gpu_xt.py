@@ -134,3 +134,55 @@ def test_xt_files_and_power_over_periods(cudapic, cuda_device, tmp_path):
             assert "Absorbed power calculated as <j*E>:" in text
     finally:
         st.close()
+
+
+@pytest.mark.parametrize("n_g", [3, 255, 800, 801, 1025, 4096])
+def test_grid_quantities_over_several_columns(cudapic, cuda_device, oracle, n_g):
+    """65 measured steps in a vacuum field of 250 V that changes every step:
+    potential, field and densities summed per XT column equal, bit for bit, the
+    FP64 sums of what each step leaves behind, in one call and in 65 (the same
+    particles: three electrons and an ion without gas or charge)."""
+    from cudapic_b200.sim import GpuSimState, ParticlesSoA
+    from gpu_util import device_array
+    steps, n_t = 65, 4000
+    params = cudapic.default_params(capacity=64, n_g=n_g, pressure=1e-9, weight=1e-20, n_t=n_t)
+    x = np.array([0.0070, 0.0125, 0.0190], np.float32)
+    v = np.zeros((3, 3), np.float32)
+    got, raw = [], None
+    for calls in (1, steps):
+        st = GpuSimState(params)
+        st.upload_electrons(ParticlesSoA(x, *v))
+        st.upload_ions(ParticlesSoA(x[:1], *v[:, :1]))
+        st.seed()
+        st.set_measure(True)
+        n_xt = st.xt_shape()[1]
+        if calls == 1:
+            st.run_steps(steps)
+        else:
+            raw = {k: np.zeros((n_g, n_xt)) for k in ("pot", "efield", "ne", "ni", "count_e", "ue", "meanee", "ioniz",
+                                                      "count_i", "ui", "meanei")}
+            before, ion = (np.zeros(n_g), np.zeros(n_g)), None
+            for t in range(steps):
+                st.run_steps(1)
+                st.synchronize()
+                b = st.buffers()
+                c = t // 20
+                raw["pot"][:, c] += device_array(b.pot, n_g, np.float32).astype(np.float64)
+                raw["efield"][:, c] += device_array(b.efield, n_g, np.float32).astype(np.float64)
+                ce, ci, _ = st.download_measurements()
+                if t % params.n_sub == 0:
+                    ion = (ci - before[1]).astype(np.float32).astype(np.float64)
+                raw["ne"][:, c] += (ce - before[0]).astype(np.float32).astype(np.float64)
+                raw["ni"][:, c] += ion
+                before = (ce.copy(), ci.copy())
+        assert st.counts() == (3, 1) and st.device_error() == 0
+        got.append({k: st.download_xt(k) for k in ("pot", "efield", "ne", "ni")} |
+                   {"cumul": np.stack(st.download_measurements()[:2])})
+        st.close()
+    want = oracle.xt_normalise(raw, params.n_t, n_xt, steps, params.gap, n_g, params.frequency, params.weight,
+                               params.electrode_area)
+    for name in ("pot", "efield", "ne", "ni"):
+        assert np.any(want[name])
+        np.testing.assert_array_equal(got[1][name], want[name], err_msg=name)
+        np.testing.assert_array_equal(got[0][name], got[1][name], err_msg=name)
+    np.testing.assert_array_equal(got[0]["cumul"], got[1]["cumul"])
