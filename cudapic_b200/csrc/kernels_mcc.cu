@@ -230,9 +230,11 @@ constexpr float MS_TABLE_EV = 32.7f;            // energies below have an index 
 // full test where they are: a queue's particles are gathered again, 32 at a
 // time, which pays for a few of 128 and not for a hot or strongly collisional
 // population.  2 000 001 electrons of 3 / 30 / 1000 eV (a call, 10 Pa) took 31 /
-// 82 / 118 us by the queue alone, now 31 / 43 / 42 (37 / 45 / 47 with the full
-// test on every particle); ions of 500 eV at 100 Pa, bounded, 77, now 54 (63).
-// Between the two forms the calls cross at a quarter to a half of a tile.
+// 82 / 118 us by the queue alone, now 28 / 38 / 38 (34 / 43 / 40 with the full
+// test on every particle, its table in shared memory); ions of 500 eV at 100 Pa,
+// bounded, 77, now 48 (52).  Between the two forms the calls cross at a quarter
+// to a half of a tile.  That full test stays ahead where nearly every particle
+// is tested and scatters: 30 eV at 100 / 1000 Pa 55 / 121 us, here 59 / 138.
 constexpr int MS_DENSE_E = 32, MS_DENSE_I = 48;
 
 // The larger of two floats, NaN (the canonical one, 0x7fffffff) if either is.
@@ -340,12 +342,61 @@ __global__ void __launch_bounds__(MS_THREADS, 1)
         __syncwarp();
     };
 
+    auto passes = [&](Xoshiro128p &rs, float v2) {  // the certain rejection; rs past the test's draws
+        bool p;
+        if (ION) {
+            rs.next();  // the target atom's four draws
+            rs.next();
+            rs.next();
+            rs.next();
+            p = ion_surely_passes(rs.uniform(), v2, k2, c);
+        } else {
+            p = !may_collide(rs.uniform(), v2, k2);
+        }
+        return p && (BOUNDED || v2 < v2_max);
+    };
+
     uint32_t qn = 0;  // entries in this warp's queue (warp-uniform)
+    // A thread for each particle: one per lane, so that every warp has some of
+    // the colliders.  A warp scatters 32 at a time, one lot after the other, and
+    // with tiles of 128 three quarters of the warps have none: 1000 / 20 000 /
+    // 120 000 electrons of 30 eV at 1000 Pa, a call, 33.3 / 33.0 / 36.1 us, now
+    // 20.8 / 21.3 / 24.1; of 3 eV at 10 Pa 16.2 / 17.1 / 19.4, now 16.8 / 17.0 /
+    // 17.9.
+    const bool one = n <= gridDim.x * MS_THREADS;
+    if (one) {
+        const uint32_t i = (blockIdx.x + (uint32_t)warp * gridDim.x) * 32u + (uint32_t)lane;
+        float vxi = 0.0f, vyi = 0.0f, vzi = 0.0f;
+        Xoshiro128p r0{};
+        if (i < n) {
+            vxi = vx[i], vyi = vy[i], vzi = vz[i];
+            r0 = Xoshiro128p{rng0[i], rng1[i], rng2[i], rng3[i]};
+        }
+        Xoshiro128p rs = r0;
+        const bool undecided = !passes(rs, vxi * vxi + vyi * vyi + vzi * vzi) && i < n;
+        if (i < n && !undecided) {
+            rng0[i] = rs.s0;
+            rng1[i] = rs.s1;
+            rng2[i] = rs.s2;
+            rng3[i] = rs.s3;
+            if (EVENTS) events[i] = 0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, undecided);
+        if (undecided) {
+            const uint32_t q = __popc(m & lt);
+            wq[0 * MS_QCAP + q] = i;
+            wq[1 * MS_QCAP + q] = r0.s0;
+            wq[2 * MS_QCAP + q] = r0.s1;
+            wq[3 * MS_QCAP + q] = r0.s2;
+            wq[4 * MS_QCAP + q] = r0.s3;
+        }
+        qn = __popc(m);
+    }
     // ions: this warp met a tile beyond MS_DENSE_I; its further tiles skip the bound (50 eV at 100 Pa, unbounded,
     // 54 us with it, 51 without; for electrons the flag cost 2 to 8 %)
     bool dense = false;
     // tile t to CTA t mod gridDim: every SM gets the same number to within one
-    const uint32_t tiles = (uint32_t)(((uint64_t)n + MS_TILE - 1) / MS_TILE);
+    const uint32_t tiles = one ? 0u : (uint32_t)(((uint64_t)n + MS_TILE - 1) / MS_TILE);
     for (uint32_t t = blockIdx.x + (uint32_t)warp * gridDim.x; t < tiles; t += gridDim.x * MS_WARPS) {
         const uint32_t i0 = t * MS_TILE + (uint32_t)lane * (vec ? MS_ROW : 1u);
         const bool whole = vec && n - min(n, i0) >= MS_ROW;
@@ -387,17 +438,7 @@ __global__ void __launch_bounds__(MS_THREADS, 1)
             for (int u = 0; u < MS_ROW; ++u) {
                 const float v2 = v[0][u] * v[0][u] + v[1][u] * v[1][u] + v[2][u] * v[2][u];
                 Xoshiro128p rs{s[0][u], s[1][u], s[2][u], s[3][u]};
-                bool passes;
-                if (ION) {
-                    rs.next();  // the target atom's four draws
-                    rs.next();
-                    rs.next();
-                    rs.next();
-                    passes = ion_surely_passes(rs.uniform(), v2, k2, c);
-                } else {
-                    passes = !may_collide(rs.uniform(), v2, k2);
-                }
-                if (passes && (BOUNDED || v2 < v2_max)) {
+                if (passes(rs, v2)) {
                     s[0][u] = rs.s0;
                     s[1][u] = rs.s1;
                     s[2][u] = rs.s2;

@@ -368,7 +368,8 @@ __device__ __forceinline__ float ion_bound_offset(float k, float normal_range) {
 // The full test of a lane's particles that the certain rejection left open
 // (bit u of `open`; states s[.][u] before the test): those that do not collide
 // get their advanced state and leave `open`.  Electrons two at a time: their
-// lookups together; four at a time spilled registers (3 us of 46).
+// lookups together; four at a time spilled registers (3 us of 46).  No lookups
+// for the decided ones (4 M electrons of 30 eV at 10 Pa 65.8 us with, now 59.1).
 template <typename Table>
 __device__ __forceinline__ void settle_electrons(uint32_t &open, const float (&v)[3][4], uint32_t (&s)[4][4],
                                                  const Table &sigma_tot_e, const cudapic_grid &g) {
@@ -379,7 +380,7 @@ __device__ __forceinline__ void settle_electrons(uint32_t &open, const float (&v
         for (int q = 0; q < 2; ++q) {
             const int u = h + q;
             v2[q] = v[0][u] * v[0][u] + v[1][u] * v[1][u] + v[2][u] * v[2][u];
-            sigma[q] = sigma_tot_e(energy_index(g.half_me_over_e * v2[q]));
+            sigma[q] = open >> u & 1u ? sigma_tot_e(energy_index(g.half_me_over_e * v2[q])) : 0.0f;
         }
 #pragma unroll
         for (int q = 0; q < 2; ++q) {

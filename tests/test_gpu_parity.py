@@ -701,6 +701,17 @@ def test_check_collisions_tile_edges(cudapic, K, oracle, dev_tables, tables, spe
         assert np.array_equal(_read(d)[:n].view(np.uint32), h[:n].view(np.uint32))
 
 
+@pytest.mark.parametrize("species,bounded", [("e", False), ("i", False), ("i", True)])
+@pytest.mark.parametrize("over,shifted", [(0, ()), (0, (1,)), (1, ()), (1, (2,)), (127, ()), (131, ()), (48_451, ())])
+def test_check_collisions_around_a_thread_per_particle(cudapic, K, oracle, dev_tables, tables, species, bounded, over,
+                                                       shifted):
+    """One particle per lane up to a thread for each (1024 per SM), four beyond:
+    both sides of the line and the ragged tiles behind it."""
+    import torch
+    n = 1024 * torch.cuda.get_device_properties(0).multi_processor_count + over
+    test_check_collisions_tile_edges(cudapic, K, oracle, dev_tables, tables, species, bounded, n, shifted)
+
+
 @pytest.mark.parametrize("species", ["e", "i"])
 @pytest.mark.parametrize("entry", [-0.0, -1e-30, -5e4, np.nan, -np.nan, np.inf])
 def test_check_collisions_odd_table_entry(cudapic, K, oracle, dev_tables, tables, species, entry):
