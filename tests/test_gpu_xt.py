@@ -186,3 +186,37 @@ def test_grid_quantities_over_several_columns(cudapic, cuda_device, oracle, n_g)
         np.testing.assert_array_equal(got[1][name], want[name], err_msg=name)
         np.testing.assert_array_equal(got[0][name], got[1][name], err_msg=name)
     np.testing.assert_array_equal(got[0]["cumul"], got[1]["cumul"])
+
+
+@pytest.mark.parametrize("over", [-3, 0, 1, 30_003])
+def test_particle_sums_around_a_thread_per_particle(cudapic, cuda_device, oracle, tables, over):
+    """The first measured step with as many particles as the grid's threads
+    (1024 per SM: one per thread, beyond that four), and on both sides: the
+    particle quantities of column 0 against the oracle (f32 partial sums per
+    CTA of a few terms per node: 2e-5, as for smaller populations)."""
+    import torch
+    from gpu_util import device_array
+    n = 1024 * torch.cuda.get_device_properties(0).multi_processor_count + over
+    st, e, i = _state(n)
+    try:
+        st.set_measure(True)
+        st.run_steps(1)
+        st.synchronize()
+        n_g, n_xt = st.xt_shape()
+        ef = device_array(st.buffers().efield, n_g, np.float32)
+        ph = oracle.phys_from_params(capacity=2 * n, weight=7.0e4 * 120000 / n)
+        re = oracle.xt_accumulate(ef, *e, False, tables[0].reshape(5, -1)[2], ph)
+        ri = oracle.xt_accumulate(ef, *i, True, None, ph)
+        raw = dict(zip(("count_e", "ue", "meanee", "ioniz", "count_i", "ui", "meanei"), tuple(re) + tuple(ri)))
+        cumul_e, cumul_i, _ = st.download_measurements()
+        raw |= {"ne": np.asarray(cumul_e), "ni": np.asarray(cumul_i), "pot": np.zeros(n_g), "efield": np.zeros(n_g)}
+        raw = {k: np.stack([v] + [np.zeros_like(v)] * (n_xt - 1), axis=1) for k, v in raw.items()}
+        p = st.params
+        want = oracle.xt_normalise(raw, p.n_t, n_xt, 1, p.gap, p.n_g, p.frequency, p.weight, p.electrode_area)
+        for name in ("je", "ji", "meanee", "meanei", "ioniz"):
+            got = st.download_xt(name)
+            scale = float(np.abs(want[name]).max())
+            assert scale > 0, name
+            np.testing.assert_allclose(got, want[name], rtol=2e-5, atol=2e-5 * scale, err_msg=name)
+    finally:
+        st.close()
